@@ -83,7 +83,16 @@ __global__ void __launch_bounds__(EpsTile::THREADS) k_eps_f64(const double* __re
 }
 
 void launch_eps_fp64(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw,
-                     double* eps, int ldn, size_t eps_stride) {
+                     double* eps, int ldn, size_t eps_stride, int smooth) {
+  // The integer tensor pipe from where it is the faster one: with 24
+  // frequencies P0 took 137 (DMMA) and 152 us (digits) at naux 300 / nov 949,
+  // 295 and 209 us at 350 / 1411, 474 and 264 us at 423 / 2020.  Its digits are
+  // relative to the largest entry of a row of B_ov chi': only for weights that
+  // do not differ too much (smooth), and for K long enough for its error (which
+  // grows as sqrt(K), the DMMA's as K) to be the smaller one in any case.
+  if (smooth && naux >= 256 && nov >= 1024 &&
+      launch_eps_digits(ctx, bov, ldov, naux, nov, chi, nw, eps, ldn, eps_stride))
+    return;
   using T = EpsTile;
   const int tiles = ceil_div(naux, T::BM);
   dim3 grid(tiles * (tiles + 1) / 2, nw);
@@ -1236,6 +1245,13 @@ __global__ void __launch_bounds__(PairTile::THREADS) k_pair_contract_f64(const d
 
 void launch_pair_contract_fp64(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc,
                                int ldn, size_t wc_stride, int nw, double* v, int ldv) {
+  // The integer tensor pipe above one column tile: with 24 frequencies the
+  // contraction took 44 (DMMA) and 32 us (digits) at naux 139 with 160 pairs,
+  // 72 and 35 us at naux 196 with 224, 178 and 84 us with 3136; at naux 86 the
+  // DMMA kernel was the faster one (24 against 27 us).  Its four launches more
+  // cost ~12 us on the host, so the line is drawn at 160.
+  if (naux > 160 && launch_pair_contract_digits(ctx, bpt, ldk, npair, naux, wc, ldn, wc_stride, nw, v, ldv))
+    return;
   using T = PairTile;
   static PerDeviceOnce attr_once;
   attr_once(ctx->device, [&] {

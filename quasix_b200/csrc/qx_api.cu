@@ -315,7 +315,8 @@ void gw_wc_p0(qx_ctx* ctx, GWSystem& S, const double* e_host) {
     launch_eps_tc(ctx, S.bov, S.ldov, S.naux, S.nov, S.chi, S.nw, S.eps, S.ldn, S.eps_stride,
                   S.precision == QX_PREC_FP16X3);
   else
-    launch_eps_fp64(ctx, S.bov, S.ldov, S.naux, S.nov, S.chi, S.nw, S.eps, S.ldn, S.eps_stride);
+    launch_eps_fp64(ctx, S.bov, S.ldov, S.naux, S.nov, S.chi, S.nw, S.eps, S.ldn, S.eps_stride,
+                    chi_smooth(e_host, S.nocc, S.nvir, 0.0));
   record_stage(ctx, QX_ST_P0, false);
 }
 
@@ -488,6 +489,13 @@ bool eps_at_least_identity(const double* energies, int nocc, int nvir, double wm
   for (int a = 0; a < nvir; ++a) lumo = std::min(lumo, energies[nocc + a]);
   const double gap = lumo - homo;
   return std::isfinite(gap) && gap > 0.0 && gap > std::fabs(wmax);
+}
+
+bool chi_smooth(const double* energies, int nocc, int nvir, double wmax) {
+  if (!eps_at_least_identity(energies, nocc, nvir, wmax / 0.9)) return false;
+  const auto occ = std::minmax_element(energies, energies + nocc);
+  const auto vir = std::minmax_element(energies + nocc, energies + nocc + nvir);
+  return *vir.second - *occ.first <= 64.0 * (*vir.first - *occ.second);
 }
 
 void validate_common(int nmo, int nocc, int naux) {
@@ -688,9 +696,12 @@ qx_status qx_get_rho_response(qx_ctx* ctx, int nfreq, const double* freqs, const
     ctx->ws[WS_EPS].reserve((size_t)nfreq * stride * sizeof(double));
     double* eps = ctx->ws[WS_EPS].as<double>();
     launch_chi(ctx, d_e, nocc, nvir, d_f, nfreq, 0, chi, ldov);
+    std::vector<double> e(nocc + nvir);
+    QX_CUDA(cudaMemcpy(e.data(), mo_energy, e.size() * sizeof(double), cudaMemcpyDefault));
     if (is_tc_precision(precision))
       launch_eps_tc(ctx, bov, ldov, naux, nov, chi, nfreq, eps, ldn, stride, precision == QX_PREC_FP16X3);
-    else launch_eps_fp64(ctx, bov, ldov, naux, nov, chi, nfreq, eps, ldn, stride);
+    else
+      launch_eps_fp64(ctx, bov, ldov, naux, nov, chi, nfreq, eps, ldn, stride, chi_smooth(e.data(), nocc, nvir, 0.0));
     // Pi = I - eps.
     std::vector<double> h((size_t)nfreq * stride);
     QX_CUDA(cudaMemcpyAsync(h.data(), eps, h.size() * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));

@@ -285,8 +285,10 @@ void CdEngine::residue_p0(CdResidueChunk& c, const CdResidue* list, int rc) {
   const size_t stride = (size_t)naux * ldn;
   std::vector<double> wr(rc);
   std::vector<int2> nm(rc);
+  double wmax = 0.0;
   for (int r = 0; r < rc; ++r) {
     wr[r] = list[r].w;
+    wmax = std::max(wmax, std::fabs(list[r].w));
     nm[r] = make_int2(tg[list[r].t], list[r].m);
   }
   QX_CUDA(cudaMemcpyAsync(c.wr, wr.data(), rc * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
@@ -297,7 +299,7 @@ void CdEngine::residue_p0(CdResidueChunk& c, const CdResidue* list, int rc) {
     launch_eps_tc(ctx, S.bov, S.ldov, naux, nov, c.chi, rc, c.eps, ldn, stride, precision == QX_PREC_FP16X3,
                   /*reuse_a=*/1);
   else
-    launch_eps_fp64(ctx, S.bov, S.ldov, naux, nov, c.chi, rc, c.eps, ldn, stride);
+    launch_eps_fp64(ctx, S.bov, S.ldov, naux, nov, c.chi, rc, c.eps, ldn, stride, chi_smooth(e.data(), nocc, nvir, wmax));
 }
 
 void CdEngine::residue_post(CdResidueChunk& c, int rc, bool refine) {
@@ -598,7 +600,9 @@ qx_ctx* make_worker(int device) {
 static double cd_system_bytes(const qx_cd_system& s, int nw, bool tc) {
   const double ldn = round_up(s.naux, 8), nov = (double)s.nocc * (s.nmo - s.nocc), ldov = round_up((int)nov, 8);
   const double eps = (nw + 2.0 * s.ntarget) * s.naux * ldn * 8.0;
-  const double p0 = s.naux * ldov * 8.0 + nw * ldov * 8.0 + (tc ? (1.0 + nw) * s.naux * ldov * 4.0 : 0.0);
+  // FP64: the digits of B_ov and of a chunk of its chi-scaled copies (k_digits.cu).
+  const double digits = 7.0 * s.naux * ldov + std::min(512.0 * 1048576, 7.0 * nw * s.naux * ldov);
+  const double p0 = s.naux * ldov * 8.0 + nw * ldov * 8.0 + (tc ? (1.0 + nw) * s.naux * ldov * 4.0 : digits);
   const double pairs = (double)s.ntarget * s.nmo * ldn * (tc ? 16.0 : 8.0) + nw * (double)s.ntarget * s.nmo * 8.0;
   return eps + p0 + nov * ldn * 8.0 + pairs;
 }

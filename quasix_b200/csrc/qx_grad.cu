@@ -338,7 +338,8 @@ extern "C" qx_status qx_g0w0_cd_grad(qx_ctx* ctx, const double* mo_energy, const
       if (E.tc)
         launch_eps_tc(ctx, E.S.bov, ldov, naux, nov, chi, fc, eps, ldn, stride, precision == QX_PREC_FP16X3);
       else
-        launch_eps_fp64(ctx, E.S.bov, ldov, naux, nov, chi, fc, eps, ldn, stride);
+        launch_eps_fp64(ctx, E.S.bov, ldov, naux, nov, chi, fc, eps, ldn, stride,
+                        chi_smooth(E.e.data(), nocc, nvir, 0.0));
       launch_invert_wc(ctx, eps, naux, ldn, stride, fc, !eps_at_least_identity(E.e.data(), nocc, nvir, 0.0), 0,
                        /*split_update=*/E.tc);
       // Y[f][p] = Wc_f b_p

@@ -168,6 +168,7 @@ enum WsSlot {
   WS_GRAD0, WS_GRAD1, WS_GRAD2,  // CD adjoint: accumulators, per-frequency chunk, lpq gradient
   WS_SWEEP_SPLIT,  // split sweep panels (two steps in flight)
   WS_GUARD,        // guarded inversion: copies of eps and the pivoted fallback's work arrays
+  WS_DIG_A, WS_DIG_B, WS_DIG_S, WS_DIG_P,  // digit operands, their scales, row-dot partial sums
   WS_COUNT
 };
 static_assert(WS_COUNT <= 40, "workspace slots");
@@ -243,9 +244,23 @@ void scaled_legendre_roots(int nw, double x0, double* freqs, double* wts);
 void launch_chi(qx_ctx* ctx, const double* energies, int nocc, int nvir, const double* freqs, int nw,
                 int real_axis, double* chi, int ldov);
 
-// eps[w] = I + B_ov diag(chi'[w]) B_ov^T for nw frequencies (FP64).
+// eps[w] = I + B_ov diag(chi'[w]) B_ov^T for nw frequencies (FP64).  smooth:
+// chi' is positive and its entries differ by a bounded factor (chi_smooth).
 void launch_eps_fp64(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw,
-                     double* eps, int ldn, size_t eps_stride);
+                     double* eps, int ldn, size_t eps_stride, int smooth);
+
+// The chi' of these energies (host array) are all positive and within a factor
+// of about 64 of each other, on the imaginary axis (wmax = 0) or for real
+// shifts up to wmax: every shift stays below 0.9 of the smallest transition and
+// the largest transition is at most 64 times the smallest.
+bool chi_smooth(const double* energies, int nocc, int nvir, double wmax);
+
+// The FP64 contractions on the integer tensor pipe (k_digits.cu); false when
+// the device has no room for their operands (nothing was done).
+bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw,
+                       double* eps, int ldn, size_t eps_stride);
+bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc,
+                                 int ldn, size_t wc_stride, int nw, double* v, int ldv);
 
 // ---------------------------------------------------------------------------
 // Guarded inversion (k_pivot.cu).  The block sweep has no pivoting; when eps
