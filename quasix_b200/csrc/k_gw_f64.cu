@@ -125,89 +125,108 @@ void launch_eps_fp64(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov
 constexpr int SWEEP_NB = 128;
 
 // The kb x kb diagonal block, padded with the identity to 128 x 128, is swept
-// in four sub-blocks of 32 (the block sweep applied recursively): warp 0 sweeps
-// the 32 x 32 sub-block element by element in registers (lane j holds column
-// j; pivot rows and columns travel by shuffles, so a pivot step costs no block
-// barrier), then the whole CTA applies the rank-32 update to the rest of the
-// 128 x 128 block through shared memory.
+// in four sub-blocks of 32 (the block sweep applied recursively): four warps,
+// one per scheduler, sweep the 32 x 32 sub-block element by element in
+// registers, then the whole CTA applies the rank-32 update to the rest of the
+// 128 x 128 block on the FP64 tensor pipe.
+//
+// What bounds it is the chain of 128 pivots: at 32 frequencies 32 CTAs run, one
+// per matrix.  A step of the chain is a division, the hand over of the pivot
+// row through shared memory (one barrier of 128 threads), a multiplication and
+// an FMA.  With all 32 rows in one warp (62 shuffles and 62 FMAs to issue per
+// pivot, 625 cycles) and the rank-32 updates by FMAs, a 128-wide block took 65
+// us; four warps that took the pivot column by shuffles 430 cycles per pivot;
+// the column is read from the pivot row instead, S being symmetric.  Eight
+// steps by the warp that holds their rows with one barrier per eight measured
+// slower (the other warps' eight steps then follow in series).
+// kDiagLd: row stride of the block in shared memory, 4 doubles past a multiple
+// of 16 for conflict-free DMMA fragments.
+constexpr int kDiagLd = SWEEP_NB + 4;
+constexpr int kDiagSmem = (SWEEP_NB * kDiagLd + 2 * 34) * (int)sizeof(double);
+
+// Warps 0..3: rows 8 warp .. 8 warp + 7 of the sub-block, lane = column.
+// prow: [2][34] doubles, the pivot row and 1 / pivot by the parity of the step.
 // A pivot at or below tol (0 unguarded: an exact zero), or a non-finite one,
 // sets bad_any.  GUARD: gm also takes max |entry| of the columns not yet
-// swept after each pivot step (the element growth of the elimination).
+// swept, sampled every eighth pivot (the probe backward error of the guard
+// catches any loss between samples).
 template <bool GUARD>
-__device__ __forceinline__ void sweep32_warp(double* S, int q0, int lane, bool& bad_any, double tol, double& gm) {
-  // Four pivot steps per loop iteration: at the start of group p4, c[k]
-  // holds S[(p4 + k) % 32][lane], so step s's pivot row is c[s] and every
-  // register index is a compile-time constant; the array then rotates by four
-  // (an unrolled loop of 32 steps measured slower, it misses the instruction
-  // cache; one step per iteration spent 64 register moves per pivot on the
-  // rotation).  The lanes other than p take c[k] - S[r][p] S[p][lane] / d and
-  // lane p takes S[r][p] / d, both as one FMA: fma(ck, b, c[k] * a) with
-  // (a, b) = (1, -rj) or (0, inv).
-  double c[32];
+__device__ __forceinline__ void sweep32_warps(double* S, double* prow, int q0, int warp, int lane, bool& bad_any,
+                                              double tol, double& gm) {
+  double c[8];
 #pragma unroll
-  for (int i = 0; i < 32; ++i) c[i] = S[(q0 + i) * SWEEP_NB + q0 + lane];
-  constexpr int UNR = 4;
+  for (int i = 0; i < 8; ++i) c[i] = S[(q0 + 8 * warp + i) * kDiagLd + q0 + lane];
 #pragma unroll 1
-  for (int p4 = 0; p4 < 32; p4 += UNR) {
+  for (int w8 = 0; w8 < 4; ++w8) {
+    const bool own = warp == w8;
 #pragma unroll
-    for (int s = 0; s < UNR; ++s) {
-      const int p = p4 + s;
-      const double d = __shfl_sync(0xffffffffu, c[s], p);
-      const bool bad = !(fabs(d) > tol) || !isfinite(d);
-      bad_any |= bad;
-      const double inv = bad ? 0.0 : 1.0 / d;
-      const double rj = c[s] * inv;  // S[p][lane] / d
-      const bool piv = (lane == p);
-      const double a = piv ? 0.0 : 1.0, b = piv ? inv : -rj;
-#pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        if (k == s) continue;
-        const double ck = __shfl_sync(0xffffffffu, c[k], p);  // S[row k][p]
-        c[k] = fma(ck, b, c[k] * a);
+    for (int s = 0; s < 8; ++s) {
+      const int p = 8 * w8 + s;
+      double* pr = prow + (s & 1) * 34;
+      if (own) {
+        const double d = __shfl_sync(0xffffffffu, c[s], p);
+        const bool bad = !(fabs(d) > tol) || !isfinite(d);
+        bad_any |= bad;
+        const double inv = bad ? 0.0 : 1.0 / d;
+        pr[lane] = c[s];
+        if (lane == 0) pr[32] = inv;
       }
-      c[s] = piv ? -inv : rj;
-      // Growth of the columns not yet swept, sampled every eighth pivot (the
-      // serial pivot chain is this kernel's bound; the probe backward error of
-      // the guard catches any loss between samples).
-      if (GUARD && (p & 7) == 7 && lane > p) {
+      asm volatile("bar.sync 1, 128;\n" ::: "memory");
+      const double inv = pr[32], rj = pr[lane] * inv;  // S[p][lane] / d
+      const bool piv = lane == p;
+      double ck[8];  // S[row k][p] = S[p][row k]
 #pragma unroll
-        for (int i = 0; i < 32; ++i) gm = fmax(gm, isfinite(c[i]) ? fabs(c[i]) : INFINITY);
+      for (int k = 0; k < 8; k += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(pr + 8 * warp + k);
+        ck[k] = v.x;
+        ck[k + 1] = v.y;
+      }
+      // The lanes other than p take c[k] - S[k][p] S[p][lane] / d, lane p S[k][p] / d.
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const double v = piv ? ck[k] * inv : fma(ck[k], -rj, c[k]);
+        c[k] = (own && k == s) ? (piv ? -inv : rj) : v;
+      }
+      if (GUARD && s == 7 && lane > p) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) gm = fmax(gm, isfinite(c[k]) ? fabs(c[k]) : INFINITY);
       }
     }
-    double t[UNR];
-#pragma unroll
-    for (int i = 0; i < UNR; ++i) t[i] = c[i];
-#pragma unroll
-    for (int i = 0; i + UNR < 32; ++i) c[i] = c[i + UNR];
-#pragma unroll
-    for (int i = 0; i < UNR; ++i) c[32 - UNR + i] = t[i];
   }
 #pragma unroll
-  for (int i = 0; i < 32; ++i) S[(q0 + i) * SWEEP_NB + q0 + lane] = c[i];
+  for (int i = 0; i < 8; ++i) S[(q0 + 8 * warp + i) * kDiagLd + q0 + lane] = c[i];
 }
 
 // D = -(A_KK)^-1 for the kb x kb diagonal block whose first element is at
 // Akk (row stride ldn), zero outside kb x kb; *status_w = 1 when a pivot is at
 // or below tol (guarded sweep) or vanishes.  growth_w (guarded sweep, else
 // null): max |A_KK| of the not-yet-swept block joins it.  512 threads;
-// dynamic shared memory (128 * 128 + 128 * 33) doubles.
+// kDiagSmem bytes of dynamic shared memory.
 __device__ __forceinline__ void block_amax(double m, double* red, unsigned long long* out);
 template <bool GUARD>
 __device__ __forceinline__ void sweep_diag_body(const double* __restrict__ Akk, int ldn, int kb,
                                                 double* __restrict__ D, int* __restrict__ status_w, double tol,
                                                 unsigned long long* growth_w) {
   static_assert(SWEEP_NB == 128, "thread mapping assumes 128 columns");
-  constexpr int TLD = 33;                       // padded row stride of T
-  extern __shared__ double S[];                 // [128][128]
-  double* Tb = S + SWEEP_NB * SWEEP_NB;         // [128][33]
+  constexpr int LD = kDiagLd;
+  extern __shared__ double S[];                 // [128][LD]
+  double* prow = S + SWEEP_NB * LD;             // [2][34]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int j = tid & 127, r0 = tid >> 7;
+  const int fr = lane >> 2, fk = lane & 3;      // DMMA fragment row / k of this lane
   double gm = 0.0;  // GUARD: max |entry| met in the unswept part
-  for (int k = 0; k < 32; ++k) {
-    const int i = r0 + 4 * k;
-    const double v = (i < kb && j < kb) ? Akk[(size_t)i * ldn + j] : (i == j ? 1.0 : 0.0);
-    S[i * SWEEP_NB + j] = v;
-    if (GUARD) gm = fmax(gm, isfinite(v) ? fabs(v) : INFINITY);
+  // Akk is 16-byte aligned (block columns and row strides are multiples of 8).
+#pragma unroll 8
+  for (int k = 0; k < 16; ++k) {
+    const int i = (tid >> 6) + 8 * k, j = 2 * (tid & 63);
+    double2 v = make_double2(0.0, 0.0);
+    if (i < kb && j + 1 < kb)
+      v = *reinterpret_cast<const double2*>(Akk + (size_t)i * ldn + j);
+    else if (i < kb && j < kb)
+      v.x = Akk[(size_t)i * ldn + j];
+    if (i >= kb || j >= kb) v.x = i == j ? 1.0 : 0.0;
+    if (i >= kb || j + 1 >= kb) v.y = i == j + 1 ? 1.0 : 0.0;
+    *reinterpret_cast<double2*>(S + i * LD + j) = v;
+    if (GUARD) gm = fmax(gm, isfinite(v.x) && isfinite(v.y) ? fmax(fabs(v.x), fabs(v.y)) : INFINITY);
   }
   bool bad_any = false;
   // Sub-blocks past kb are identity padding with no coupling to the block:
@@ -217,103 +236,80 @@ __device__ __forceinline__ void sweep_diag_body(const double* __restrict__ Akk, 
   for (int sb = 0; sb < nsb; ++sb) {
     const int q0 = 32 * sb;
     __syncthreads();
-    if (warp == 0) sweep32_warp<GUARD>(S, q0, lane, bad_any, tol, gm);
+    if (warp < 4) sweep32_warps<GUARD>(S, prow, q0, warp, lane, bad_any, tol, gm);
     __syncthreads();
-    // Both products below use register tiles (thread = 4 rows x 2 or 8
-    // columns), so each shared-memory operand feeds several FMAs.
-    const int rt = tid >> 4, ct = tid & 15, rb = 4 * rt;
-    // T[r][q] = S[r][Q] D1 = -S[r][Q] Sswept[Q][q] for rows outside Q (0 inside).
+    // The twelve 8-row tiles outside Q: tile i starts at row out(i).
+    auto out = [&](int i) { return 8 * (i < 4 * sb ? i : i + 4); };
+    // T[r][q] = S[r][Q] D1 = -S[r][Q] Sswept[Q][q] for the rows outside Q, in
+    // place: warp -> 8 columns and three row tiles.
     {
-      const int cb = 2 * ct;
-      double t[4][2];
+      const int n0 = 8 * (warp & 3);
+      double acc[3][2] = {};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) t[i][0] = t[i][1] = 0.0;
-#pragma unroll 4
-      for (int p = 0; p < 32; ++p) {
-        const double b0 = S[(q0 + p) * SWEEP_NB + q0 + cb], b1 = S[(q0 + p) * SWEEP_NB + q0 + cb + 1];
+      for (int p = 0; p < 32; p += 4) {
+        const double b = S[(q0 + p + fk) * LD + q0 + n0 + fr];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const double a = S[(rb + i) * SWEEP_NB + q0 + p];
-          t[i][0] -= a * b0;
-          t[i][1] -= a * b1;
-        }
+        for (int i = 0; i < 3; ++i) dmma_8x8x4(acc[i], S[(out(3 * (warp >> 2) + i) + fr) * LD + q0 + p + fk], b);
       }
+      __syncthreads();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const bool inq = (rb + i >= q0 && rb + i < q0 + 32);
-        Tb[(rb + i) * TLD + cb] = inq ? 0.0 : t[i][0];
-        Tb[(rb + i) * TLD + cb + 1] = inq ? 0.0 : t[i][1];
-      }
+      for (int i = 0; i < 3; ++i)
+        *reinterpret_cast<double2*>(S + (out(3 * (warp >> 2) + i) + fr) * LD + q0 + n0 + 2 * fk) =
+            make_double2(-acc[i][0], -acc[i][1]);
     }
     __syncthreads();
     // S[r][c] -= T[r] . S[Q][c]  for r, c outside Q (old S[Q][c]; rows in Q
-    // are read, never written here).
+    // are read, never written here): warp -> 3 x 3 tiles of 8 x 8.
     {
-      // Columns 32 v + 2 ct + {0, 1}, v = 0..3: a warp's double2 loads are
-      // contiguous (conflict-free), and each 32-column group lies wholly
-      // inside or outside Q.
-      const int cb = 2 * ct;
-      double acc[4][8];
+      double acc[3][3][2] = {};
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int p = 0; p < 32; p += 4) {
+        double a[3], b[3];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) acc[i][c] = 0.0;
-#pragma unroll 2
-      for (int p = 0; p < 32; ++p) {
-        double bv[8];
-        const double* brow = S + (q0 + p) * SWEEP_NB + cb;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const double2 x2 = *reinterpret_cast<const double2*>(brow + 32 * v);
-          bv[2 * v] = x2.x;
-          bv[2 * v + 1] = x2.y;
+        for (int i = 0; i < 3; ++i) {
+          a[i] = S[(out(3 * (warp >> 2) + i) + fr) * LD + q0 + p + fk];
+          b[i] = S[(q0 + p + fk) * LD + out(3 * (warp & 3) + i) + fr];
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const double a = Tb[(rb + i) * TLD + p];
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-          for (int c = 0; c < 8; ++c) acc[i][c] += a * bv[c];
-        }
+          for (int k = 0; k < 3; ++k) dmma_8x8x4(acc[i][k], a[i], b[k]);
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (rb + i >= q0 && rb + i < q0 + 32) continue;
+      for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          if (32 * v == q0) continue;
-          const double s0 = S[(rb + i) * SWEEP_NB + 32 * v + cb] - acc[i][2 * v];
-          const double s1 = S[(rb + i) * SWEEP_NB + 32 * v + cb + 1] - acc[i][2 * v + 1];
-          S[(rb + i) * SWEEP_NB + 32 * v + cb] = s0;
-          S[(rb + i) * SWEEP_NB + 32 * v + cb + 1] = s1;
+        for (int k = 0; k < 3; ++k) {
+          const int r = out(3 * (warp >> 2) + i) + fr, cc = out(3 * (warp & 3) + k) + 2 * fk;
+          double2* at = reinterpret_cast<double2*>(S + r * LD + cc);
+          const double s0 = at->x - acc[i][k][0], s1 = at->y - acc[i][k][1];
+          *at = make_double2(s0, s1);
           // Rows and columns past this sub-block: the Schur complement.
-          if (GUARD && rb + i >= q0 + 32 && 32 * v > q0) {
+          if (GUARD && r >= q0 + 32 && cc >= q0 + 32) {
             gm = fmax(gm, isfinite(s0) ? fabs(s0) : INFINITY);
             gm = fmax(gm, isfinite(s1) ? fabs(s1) : INFINITY);
           }
         }
-      }
     }
     __syncthreads();
-    // S[r][Q] = T[r] (lanes along q) and S[Q][r] = T[r]^T (lanes along r).
-    for (int idx = tid; idx < SWEEP_NB * 32; idx += blockDim.x) {
-      const int r = idx >> 5, q = idx & 31;
-      if (!(r >= q0 && r < q0 + 32)) S[r * SWEEP_NB + q0 + q] = Tb[r * TLD + q];
-    }
-    for (int idx = tid; idx < SWEEP_NB * 32; idx += blockDim.x) {
-      const int q = idx >> 7, r = idx & 127;
-      if (!(r >= q0 && r < q0 + 32)) S[(q0 + q) * SWEEP_NB + r] = Tb[r * TLD + q];
+    // S[Q][r] = T[r]^T, in 4 x 4 blocks per half warp (no bank conflicts on either side).
+    for (int blk = tid >> 4; blk < 8 * 24; blk += 32) {
+      const int r = out(blk >> 4) + 4 * ((blk >> 3) & 1) + (lane & 3), q = q0 + 4 * (blk & 7) + ((lane >> 2) & 3);
+      S[q * LD + r] = S[r * LD + q];
     }
   }
   __syncthreads();
-  if (lane == 0 && warp == 0 && bad_any) atomicExch(status_w, 1);
+  if (lane == 0 && warp < 4 && bad_any) atomicExch(status_w, 1);
   if (GUARD && growth_w) {
     __shared__ double gred[16];
     block_amax(gm, gred, growth_w);
   }
   // D = -S, zero outside the kb x kb block.
-  for (int k = 0; k < 32; ++k) {
-    const int i = r0 + 4 * k;
-    D[(size_t)i * SWEEP_NB + j] = (i < kb && j < kb) ? -S[i * SWEEP_NB + j] : 0.0;
+#pragma unroll 8
+  for (int k = 0; k < 16; ++k) {
+    const int i = (tid >> 6) + 8 * k, j = 2 * (tid & 63);
+    const double2 v = *reinterpret_cast<const double2*>(S + i * LD + j);
+    *reinterpret_cast<double2*>(D + (size_t)i * SWEEP_NB + j) =
+        make_double2(i < kb && j < kb ? -v.x : 0.0, i < kb && j + 1 < kb ? -v.y : 0.0);
   }
 }
 
@@ -560,7 +556,7 @@ __global__ void k_gsweep_update(const GMat* __restrict__ mats, const int* __rest
                                 const double* __restrict__ Tcat, const double* __restrict__ Pcat);
 
 void sweep_set_attributes() {
-  const int diag_smem = (int)((SWEEP_NB * SWEEP_NB + SWEEP_NB * 33) * sizeof(double));
+  const int diag_smem = kDiagSmem;
   QX_CUDA(cudaFuncSetAttribute(k_sweep_diag<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem));
   QX_CUDA(cudaFuncSetAttribute(k_sweep_diag<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem));
   QX_CUDA(cudaFuncSetAttribute(k_sweep_tpanel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PanelTile::SMEM));
@@ -587,7 +583,7 @@ static void sweep_front(qx_ctx* ctx, cudaStream_t st, double* eps, int n, int ld
                         const GuardSet* gs = nullptr) {
   if (amax_t) QX_CUDA(cudaMemsetAsync(amax_t, 0, nw * sizeof(unsigned long long), st));
   if (amax_p) QX_CUDA(cudaMemsetAsync(amax_p, 0, nw * sizeof(unsigned long long), st));
-  const int diag_smem = (SWEEP_NB * SWEEP_NB + SWEEP_NB * 33) * sizeof(double);
+  const int diag_smem = kDiagSmem;
   unsigned long long* gamax = gs ? gs->amax : nullptr;
   unsigned long long* growth = gs ? gs->growth : nullptr;
   if (gs)
@@ -952,7 +948,7 @@ void launch_invert_wc_group(qx_ctx* ctx, const GMat* mats_in, int G, int half_lo
   sweep_attributes_once(ctx->device);
   k_gzero_pad<<<G, 256, 0, ctx->stream>>>(d_mats, Tcat, Pcat);
   check_launch(ctx);
-  const int diag_smem = (SWEEP_NB * SWEEP_NB + SWEEP_NB * 33) * sizeof(double);
+  const int diag_smem = kDiagSmem;
   for (int s = 0; s < nsteps; ++s) {
     const int k0 = s * SWEEP_NB, a = act[s];
     if (guarded)
