@@ -1,8 +1,9 @@
 // BSE-TDA on the GPU: the matrix-free Hamiltonian of BSETDAKernel
 // (quasix_core/src/bse/kernel.rs:501-598) as batched GEMMs, and the block
 // Davidson of davidson_bse (quasix_core/src/bse/davidson.rs:372-508) with the
-// subspace, Rayleigh-Ritz (parallel Jacobi) and re-orthonormalisation on the
+// subspace, Rayleigh-Ritz step and re-orthonormalisation on the
 // device; the host only steers (convergence flags, subspace size).
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -10,6 +11,7 @@
 #include <cmath>
 #include <functional>
 #include <numeric>
+#include <type_traits>
 
 #include "qx_blas.cuh"
 #include "qx_internal.cuh"
@@ -73,69 +75,197 @@ __global__ void k_bse_combine(const double* __restrict__ X, const double* __rest
   }
 }
 
-// R[r] = AX[r] - theta[r] X[r]; nrm2[r] = |R[r]|^2
-__global__ void k_residual(const double* __restrict__ AX, const double* __restrict__ X, const double* __restrict__ theta,
-                           int ld, int n, double* __restrict__ R, double* __restrict__ nrm2) {
-  const int r = blockIdx.y;
-  double s = 0.0;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const double v = AX[(size_t)r * ld + k] - theta[r] * X[(size_t)r * ld + k];
-    R[(size_t)r * ld + k] = v;
-    s += v * v;
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __shared__ double red[32];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[i];
-    atomicAdd(nrm2 + r, t);
+// Ritz vectors and residuals of a Davidson step: X[r] = sum_i Z[i][r] V[i],
+// AX[r] likewise, R[r] = AX[r] - theta[r] X[r], and this block's part of |R[r]|^2
+// in nrm[blockIdx.x][r].  32 columns per block, lanes along them, the rows i
+// over eight warps and then summed in a fixed order; RB roots at a time.
+// (Two combination kernels whose blocks walked all rows i in series, then a
+// residual in one block per root, took ~40 us per step at n = 3264.)
+constexpr int kRitzRoots = 4;
+__global__ void __launch_bounds__(256) k_ritz(const double* __restrict__ V, const double* __restrict__ AV, int ld,
+                                              int nv, const double* __restrict__ Z, int ldz, int nr, int n,
+                                              const double* __restrict__ theta, double* __restrict__ X,
+                                              double* __restrict__ AX, double* __restrict__ R,
+                                              double* __restrict__ nrm) {
+  constexpr int RB = kRitzRoots;
+  __shared__ double part[8][2 * RB][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * 32 + lane;
+  for (int r0 = 0; r0 < nr; r0 += RB) {
+    double x[RB], ax[RB];
+#pragma unroll
+    for (int r = 0; r < RB; ++r) x[r] = ax[r] = 0.0;
+    if (c < n) {
+#pragma unroll 4
+      for (int i = warp; i < nv; i += 8) {
+        const double v = V[(size_t)i * ld + c], av = AV[(size_t)i * ld + c];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+          const double z = r0 + r < nr ? __ldg(Z + (size_t)i * ldz + r0 + r) : 0.0;
+          x[r] = fma(z, v, x[r]);
+          ax[r] = fma(z, av, ax[r]);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+      part[warp][r][lane] = x[r];
+      part[warp][RB + r][lane] = ax[r];
+    }
+    __syncthreads();
+    if (warp < RB && r0 + warp < nr) {
+      double xs = 0.0, as = 0.0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        xs += part[q][warp][lane];
+        as += part[q][RB + warp][lane];
+      }
+      const int r = r0 + warp;
+      double v = 0.0;
+      if (c < n) {
+        v = as - theta[r] * xs;
+        X[(size_t)r * ld + c] = xs;
+        AX[(size_t)r * ld + c] = as;
+        R[(size_t)r * ld + c] = v;
+      }
+      v *= v;
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) nrm[(size_t)blockIdx.x * nr + r] = v;
+    }
+    __syncthreads();
   }
 }
 
-// t = r / (delta - theta + shift) with the reference's clamp (davidson.rs:194-225); nrm2 += |t|^2
-__global__ void k_precond(const double* __restrict__ R, const double* __restrict__ delta, double theta, double shift,
-                          int n, double* __restrict__ t, double* __restrict__ nrm2) {
-  double s = 0.0;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    double den = delta[k] - theta + shift;
-    if (fabs(den) < 1e-8) den = (den >= 0.0) ? 1e-8 : -1e-8;
-    const double v = R[k] / den;
-    t[k] = v;
-    s += v * v;
+// Extends the orthonormal rows V[0 .. nv) by up to count candidates, one after
+// the other, each normalised, orthogonalised twice against all rows before it
+// (davidson.rs:240-285) and dropped when what is left is below lindep;
+// *added (zero on entry to the first call of a step) counts the rows gained,
+// which follow V[nv].  Candidate q is src[idx[q]], divided by delta - theta[q] +
+// shift with the reference's clamp (davidson.rs:194-225) when delta is given.
+// A cooperative launch: the blocks share the columns, and meet at a grid
+// barrier after each set of partial dot products (two per candidate), which
+// every block then adds in the same order.  STAGE: the block's columns of V are
+// kept in shared memory for the launch, so that between the barriers nothing
+// but the partial dots comes from L2.  (As separate GEMM, combination and
+// norm launches with a host decision per candidate, a step of five candidates
+// took 40 launches and five synchronisations: ~450 us at n = 3264, now 87 us.)
+constexpr int kExpandMax = 64, kExpandRed = 128, kExpandSmem = 220 * 1024;
+struct DavExpand {
+  double* V;
+  int ld, nv, n, count, cap;
+  const double* src;
+  const double* delta;
+  double shift, lindep;
+  double* part;  // [2][gridDim.x][cap + 1]
+  int* added;
+  int idx[kExpandMax];
+  double theta[kExpandMax];
+};
+template <bool STAGE>
+__global__ void __launch_bounds__(256) k_dav_expand(DavExpand a) {
+  extern __shared__ double sm[];
+  const int G = gridDim.x, g = blockIdx.x;
+  const int L = (a.n + G - 1) / G, x0 = g * L, len = max(0, min(L, a.n - x0)), ldc = a.cap + 1;
+  double* red = sm;           // [8][kExpandRed]
+  double* c = red + 8 * kExpandRed;  // [cap + 1] summed dot products
+  double* vs = c + ldc;       // [cap][L] staged rows
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  const size_t ps = (size_t)G * ldc;
+  int cur = a.nv + *a.added;
+  // The candidate's columns of this block.
+  double* t = STAGE ? vs + a.cap * L : a.V + (size_t)cur * a.ld + x0;
+  if (STAGE)
+    for (int i = warp; i < cur; i += 8)
+      for (int x = lane; x < len; x += 32) vs[i * L + x] = a.V[(size_t)i * a.ld + x0 + x];
+  const auto row = [&](int i) -> const double* { return STAGE ? vs + i * L : a.V + (size_t)i * a.ld + x0; };
+  // Dots of t with rows 0 .. cur (row cur: t itself) -> c, through part[b].
+  auto dots = [&](int b) {
+    double* out = a.part + b * ps + (size_t)g * ldc;
+    for (int i = warp; i <= cur; i += 8) {
+      double s = 0.0;
+      const double* v = i < cur ? row(i) : t;
+      for (int x = lane; x < len; x += 32) s += v[x] * t[x];
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) out[i] = s;
+    }
+    __threadfence();
+    grid.sync();
+    const double* in = a.part + b * ps;
+    for (int i0 = 0; i0 <= cur; i0 += kExpandRed) {
+      const int m = min(kExpandRed, cur + 1 - i0);
+      for (int i = lane; i < m; i += 32) {
+        double s = 0.0;
+#pragma unroll 8
+        for (int q = warp; q < G; q += 8) s += __ldcg(in + (size_t)q * ldc + i0 + i);
+        red[warp * kExpandRed + i] = s;
+      }
+      __syncthreads();
+      if (tid < m) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s += red[w * kExpandRed + tid];
+        c[i0 + tid] = s;
+      }
+      __syncthreads();
+    }
+  };
+  // t = f t - f sum_i c[i] V[i]
+  auto subtract = [&](double f) {
+    for (int xb = 0; xb < len; xb += 32) {
+      const int x = xb + lane;
+      double s = 0.0;
+      if (x < len) {
+#pragma unroll 4
+        for (int i = warp; i < cur; i += 8) s += c[i] * row(i)[x];
+      }
+      red[warp * 32 + lane] = s;
+      __syncthreads();
+      if (warp == 0 && x < len) {
+        double u = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) u += red[q * 32 + lane];
+        t[x] = f * (t[x] - u);
+      }
+      __syncthreads();
+    }
+  };
+  grid.sync();  // every block has read *added
+  for (int q = 0; q < a.count; ++q) {
+    const double* r = a.src + (size_t)a.idx[q] * a.ld + x0;
+    for (int x = tid; x < len; x += 256) {
+      double v = r[x];
+      if (a.delta) {
+        double den = a.delta[x0 + x] - a.theta[q] + a.shift;
+        if (fabs(den) < 1e-8) den = (den >= 0.0) ? 1e-8 : -1e-8;
+        v /= den;
+      }
+      t[x] = v;
+    }
+    __syncthreads();
+    dots(0);
+    const double nr = sqrt(c[cur]);
+    subtract(nr > 1e-14 ? 1.0 / nr : 1.0);
+    dots(1);
+    // |t - sum_i c[i] V[i]|^2 = |t|^2 - sum_i c[i]^2: after the first pass the
+    // c are rounding, so nothing cancels.
+    double s2 = 0.0;
+    for (int i = lane; i < cur; i += 32) s2 += c[i] * c[i];
+    for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    const double h = sqrt(fmax(c[cur] - s2, 0.0));
+    subtract(1.0);
+    if (h < a.lindep) continue;
+    const double inv = 1.0 / h;
+    for (int x = tid; x < len; x += 256) {
+      const double v = t[x] * inv;
+      a.V[(size_t)cur * a.ld + x0 + x] = v;
+      if (STAGE) vs[cur * L + x] = v;
+    }
+    __syncthreads();
+    ++cur;
+    if (!STAGE) t += a.ld;
   }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __shared__ double red[32];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double tt = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) tt += red[i];
-    atomicAdd(nrm2, tt);
-  }
-}
-
-// x[k] *= 1/sqrt(nrm2[0]) when sqrt(nrm2) > thr (thr < 0: always)
-__global__ void k_normalize(double* __restrict__ x, int n, const double* __restrict__ nrm2, double thr) {
-  const double nr = sqrt(nrm2[0]);
-  if (!(nr > thr)) return;
-  const double inv = 1.0 / nr;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) x[k] *= inv;
-}
-
-__global__ void k_norm2(const double* __restrict__ x, int n, double* __restrict__ nrm2) {
-  double s = 0.0;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) s += x[k] * x[k];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __shared__ double red[32];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[i];
-    atomicAdd(nrm2, t);
-  }
+  if (g == 0 && tid == 0) *a.added = cur - a.nv;
 }
 
 // M <- (M + M^T) / 2 for an n x n matrix (ld).
@@ -214,6 +344,11 @@ struct DevArr {
     QX_CUDA(cudaMalloc(&p, count * sizeof(double)));
     n = count;
   }
+  void free() {
+    if (p) cudaFree(p);
+    p = nullptr;
+    n = 0;
+  }
   ~DevArr() {
     if (p) cudaFree(p);
   }
@@ -221,7 +356,7 @@ struct DevArr {
 
 // Davidson subspace and scratch (grown on demand, reused across solves).
 struct DavWork {
-  DevArr V, AV, X, AX, R, heff, jv, Z2, small, eigi;
+  DevArr V, AV, X, AX, R, heff, jv, Z2, small, eigi, part;
 };
 
 struct qx_bse {
@@ -237,6 +372,10 @@ struct qx_bse {
   DevArr kd_split, kd_scale;
   int ldg = 0;
   bool kd = false;
+  // FP64: the contracted direct kernel C[(i,j)][(a,b)], formed by the first
+  // Davidson solve when it fits (ensure_kd_f64).
+  DevArr kd_f64;
+  bool kd_f64_tried = false;
   DevArr x_split;                    // split forms: hi/lo of the packed vectors
   DevArr xp, T, Yd, Z, Yx, Xr, Yr;  // matvec scratch
   DevArr gTt, gTp, gTpT, gdijT, gM, gG1, gG, gU;  // root-gradient scratch
@@ -245,6 +384,118 @@ struct qx_bse {
   std::vector<double> h_delta;
 };
 
+// Yd[i][a nvec + v] = sum_(j,b) C[(i,j)][(a,b)] X[v][(j,b)] for NV vectors from
+// v0 on.  What bounds it is reading C once (8 nov^2 bytes); each warp takes
+// KD_ROWS rows (i, a) of one i, its lanes along b, so that every C is used for
+// NV vectors and every X for KD_ROWS rows.
+constexpr int KD_ROWS = 2, KD_VECS = 6;
+template <int NV>
+__global__ void __launch_bounds__(128) k_kd_apply(const double* __restrict__ C, const double* __restrict__ X, int ldx,
+                                                  int nocc, int nvir, int nvec, int v0, double* __restrict__ Yd) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.y, a0 = (blockIdx.x * 4 + warp) * KD_ROWS;
+  if (a0 >= nvir) return;
+  const int na = min(KD_ROWS, nvir - a0);
+  double acc[KD_ROWS][NV];
+#pragma unroll
+  for (int a = 0; a < KD_ROWS; ++a)
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[a][v] = 0.0;
+  for (int j = 0; j < nocc; ++j) {
+    const double* c = C + ((size_t)(i * nocc + j) * nvir + a0) * nvir;
+    const double* x = X + (size_t)v0 * ldx + (size_t)j * nvir;
+#pragma unroll 2
+    for (int b = lane; b < nvir; b += 32) {
+      double xv[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) xv[v] = __ldg(x + (size_t)v * ldx + b);
+#pragma unroll
+      for (int a = 0; a < KD_ROWS; ++a) {
+        const double k = __ldg(c + (size_t)min(a, na - 1) * nvir + b);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) acc[a][v] = fma(k, xv[v], acc[a][v]);
+      }
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < KD_ROWS; ++a)
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      double s = acc[a][v];
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0 && a < na) Yd[((size_t)i * nvir + a0 + a) * nvec + v0 + v] = s;
+    }
+}
+
+static void kd_apply(qx_bse* B, const double* X, int nvec) {
+  qx_ctx* ctx = B->ctx;
+  const dim3 grid(ceil_div(ceil_div(B->nvir, KD_ROWS), 4), B->nocc);
+  for (int v0 = 0; v0 < nvec; v0 += KD_VECS) {
+    auto go = [&](auto nv) {
+      k_kd_apply<decltype(nv)::value><<<grid, 128, 0, ctx->stream>>>(B->kd_f64.p, X, B->ldov, B->nocc, B->nvir, nvec, v0,
+                                                                    B->Yd.p);
+    };
+    switch (std::min(KD_VECS, nvec - v0)) {
+      case 1: go(std::integral_constant<int, 1>()); break;
+      case 2: go(std::integral_constant<int, 2>()); break;
+      case 3: go(std::integral_constant<int, 3>()); break;
+      case 4: go(std::integral_constant<int, 4>()); break;
+      case 5: go(std::integral_constant<int, 5>()); break;
+      default: go(std::integral_constant<int, 6>()); break;
+    }
+    check_launch(ctx);
+  }
+}
+
+// FP64, before a Davidson solve: C[(i,j)][(a,b)] = sum_Q ijw[(i,j)][Q]
+// B_ab[(a,b)][Q] (kernel.rs:391-462 contracted once), batched over a from dabT.
+// A solve applies H a hundred times: the factored direct term costs 4 nov nvir
+// naux FLOPs per vector each time, C's one product 2 nov^2 naux FLOPs once.
+// (Dimension 3264, naux 560: 60 us against ~190 us per matvec of five vectors;
+// the product 0.8 ms.)  Held when its nov^2 doubles take at most 16 GB, the
+// bound of the split forms' K^d, and at most half of the free memory with the
+// product's operand; else, and below dimension 512, where both are a few
+// launches, the factored form stays.
+static void ensure_kd_f64(qx_bse* B) {
+  if (B->precision != QX_PREC_FP64 || B->kd_f64_tried) return;
+  B->kd_f64_tried = true;
+  const size_t n2 = (size_t)B->nov * B->nov;
+  if (B->nov < 512 || n2 * sizeof(double) > ((size_t)16 << 30)) return;
+  qx_ctx* ctx = B->ctx;
+  DevArr dab;
+  const size_t dab_n = (size_t)B->nvir * B->nvir * B->ldq;
+  size_t avail = 0, total = 0;
+  QX_CUDA(cudaMemGetInfo(&avail, &total));
+  if ((n2 + dab_n) * sizeof(double) > avail / 2) return;
+  try {
+    B->kd_f64.alloc(n2);
+    dab.alloc(dab_n);
+  } catch (const Error&) {
+    cudaGetLastError();
+    B->kd_f64.free();
+    return;
+  }
+  // dabT [a][Q][b] back to [a][b][Q].
+  QX_CUDA(cudaMemsetAsync(dab.p, 0, (size_t)B->nvir * B->nvir * B->ldq * sizeof(double), ctx->stream));
+  transpose(ctx, B->dabT.p, B->naux, B->nvir, B->ldvp, (size_t)B->naux * B->ldvp, dab.p, B->ldq,
+            (size_t)B->nvir * B->ldq, B->nvir);
+  GemmNT g{};
+  g.M = B->nocc * B->nocc;
+  g.N = B->nvir * B->nvir;
+  g.K = B->naux;
+  g.A = B->ijw.p;
+  g.lda = B->ldq;
+  g.B = dab.p;
+  g.ldb = B->ldq;
+  g.C = B->kd_f64.p;
+  g.ldc = B->nvir * B->nvir;
+  g.batch = 1;
+  g.alpha = 1.0;
+  g.splitk = 1;
+  gemm_nt_f64(ctx, g);
+  QX_CUDA(cudaStreamSynchronize(ctx->stream));  // dab is freed on return
+}
+
 // y[v] = H x[v] for nvec vectors in row layout [nvec][ldov] (device).
 // need_T: take the factored direct term even when K^d is held (the root
 // gradient reads its first step T).
@@ -252,7 +503,9 @@ static void bse_apply_rows(qx_bse* B, const double* X, double* Y, int nvec, bool
   qx_ctx* ctx = B->ctx;
   const int nocc = B->nocc, nvir = B->nvir, naux = B->naux;
   B->Yd.alloc((size_t)nocc * nvir * nvec);
-  if (B->kd && !need_T) {
+  if (B->kd_f64.p && !need_T) {
+    kd_apply(B, X, nvec);
+  } else if (B->kd && !need_T) {
     // Direct term as one GEMM: Yd[(i,a)][v] = sum_(j,b) K^d[(i,a)][(j,b)] X[v][(j,b)]
     // (the layout Yd[i][(a,v)] of the factored form).
     const int fp16 = B->precision == QX_PREC_FP16X3;
@@ -617,10 +870,14 @@ static void davidson_run(qx_ctx* ctx, DavWork& W, int n, int ld, const double* d
   W.jv.alloc(eigh_lowest_work_doubles(cap, cap));
   W.eigi.alloc(((size_t)cap * cap + 1) / 2 + 1);
   W.Z2.alloc((size_t)cap * cap);
-  W.small.alloc((size_t)4 * cap + 64);
+  const int rblk = ceil_div(n, 32);  // blocks of k_ritz
+  W.small.alloc((size_t)cap + (size_t)rblk * nroots + 64);
   double* d_theta = W.small.p;
-  double* d_nrm = d_theta + cap;
-  double* d_c = d_nrm + cap;
+  int* d_added = reinterpret_cast<int*>(d_theta + cap);
+  double* d_nrm = d_theta + cap + 8;  // [rblk][nroots]
+  // Blocks of k_dav_expand: at least 64 columns each, one per SM at most.
+  const int xblk = std::max(1, std::min(ctx->sm_count, n / 64));
+  W.part.alloc((size_t)2 * xblk * (cap + 1));
   QX_CUDA(cudaMemsetAsync(W.V.p, 0, (size_t)cap * ld * sizeof(double), ctx->stream));
   auto apply = [&](int first, int count) { apply_rows(W.V.p + (size_t)first * ld, W.AV.p + (size_t)first * ld, count); };
   auto rr = [&](int nv, int k) {
@@ -642,10 +899,50 @@ static void davidson_run(qx_ctx* ctx, DavWork& W, int n, int ld, const double* d
     gemm_nt_f64(ctx, g);
     eigh_lowest(ctx, W.heff.p, nv, nv, k, d_theta, W.Z2.p, nv, W.jv.p, reinterpret_cast<int*>(W.eigi.p));
   };
-  const int nthreads = 256, nblk = std::min(ceil_div(n, nthreads), 2 * ctx->sm_count);
-  // The norm reductions run in one block of 1024 threads each, so that their
-  // summation order (and the Davidson path) is the same on every run.
-  constexpr int kRedThreads = 1024;
+  // (Staged rows up to the limit of shared memory; beyond, V and the candidate
+  // stay in global memory.)
+  const size_t expand_base = ((size_t)8 * kExpandRed + cap + 1) * sizeof(double);
+  const size_t expand_rows = (size_t)(cap + 1) * ceil_div(n, xblk) * sizeof(double);
+  const bool stage = expand_base + expand_rows <= (size_t)kExpandSmem;
+  const size_t expand_smem = expand_base + (stage ? expand_rows : 0);
+  static PerDeviceOnce attr_once;
+  attr_once(ctx->device, [&] {
+    QX_CUDA(cudaFuncSetAttribute(k_dav_expand<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kExpandSmem));
+    QX_CUDA(cudaFuncSetAttribute(k_dav_expand<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kExpandSmem));
+  });
+  // Orthonormalise the rows list of src (preconditioned when delta is given)
+  // against and after V[0 .. nv); returns the number added (synchronises).
+  auto expand = [&](int nv, const double* src, const std::vector<int>& list, const double* delta,
+                    const std::vector<double>& theta, double lindep) {
+    QX_CUDA(cudaMemsetAsync(d_added, 0, sizeof(int), ctx->stream));
+    for (size_t q0 = 0; q0 < list.size(); q0 += kExpandMax) {
+      DavExpand a{};
+      a.V = W.V.p;
+      a.ld = ld;
+      a.nv = nv;
+      a.n = n;
+      a.cap = cap;
+      a.count = (int)std::min<size_t>(kExpandMax, list.size() - q0);
+      a.src = src;
+      a.delta = delta;
+      a.shift = cfg.level_shift;
+      a.lindep = lindep;
+      a.part = W.part.p;
+      a.added = d_added;
+      for (int q = 0; q < a.count; ++q) {
+        a.idx[q] = list[q0 + q];
+        a.theta[q] = delta ? theta[list[q0 + q]] : 0.0;
+      }
+      void* args[] = {&a};
+      QX_CUDA(cudaLaunchCooperativeKernel(stage ? (const void*)k_dav_expand<true> : (const void*)k_dav_expand<false>, dim3(xblk), dim3(256), args, expand_smem,
+                                          ctx->stream));
+      check_launch(ctx);
+    }
+    int added = 0;
+    QX_CUDA(cudaMemcpyAsync(&added, d_added, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    sync_and_check(ctx);
+    return added;
+  };
   // Trivial case (davidson.rs:384-387, 510-540): the full matrix.
   if (n <= nroots) {
     std::vector<double> id((size_t)n * ld, 0.0);
@@ -687,23 +984,23 @@ static void davidson_run(qx_ctx* ctx, DavWork& W, int n, int ld, const double* d
   QX_CUDA(cudaMemsetAsync(evecs.p, 0, (size_t)nroots * ld * sizeof(double), ctx->stream));
   int iter = 0;
   bool all = false;
-  std::vector<double> th(cap), nr(cap);
+  std::vector<double> th(cap), nr((size_t)rblk * nroots);
   for (iter = 0; iter < cfg.max_iter; ++iter) {
     const int nr_ = std::min(nroots, nv);
     rr(nv, nr_);
-    // Ritz vectors X = V Y, AX = AV Y.
-    combine_rows(ctx, W.V.p, ld, nv, W.Z2.p, nv, nr_, n, W.X.p, ld, 1.0, 0.0);
-    combine_rows(ctx, W.AV.p, ld, nv, W.Z2.p, nv, nr_, n, W.AX.p, ld, 1.0, 0.0);
-    QX_CUDA(cudaMemsetAsync(d_nrm, 0, nr_ * sizeof(double), ctx->stream));
-    k_residual<<<dim3(1, nr_), kRedThreads, 0, ctx->stream>>>(W.AX.p, W.X.p, d_theta, ld, n, W.R.p, d_nrm);
+    // Ritz vectors X = V Y, AX = AV Y and residuals.
+    k_ritz<<<rblk, 256, 0, ctx->stream>>>(W.V.p, W.AV.p, ld, nv, W.Z2.p, nv, nr_, n, d_theta, W.X.p, W.AX.p, W.R.p,
+                                          d_nrm);
     check_launch(ctx);
     QX_CUDA(cudaMemcpyAsync(th.data(), d_theta, nr_ * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    QX_CUDA(cudaMemcpyAsync(nr.data(), d_nrm, nr_ * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    QX_CUDA(cudaMemcpyAsync(nr.data(), d_nrm, (size_t)rblk * nr_ * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     sync_and_check(ctx);
     std::vector<int> newr;
     for (int j = 0; j < nroots; ++j) {
       if (j >= nr_ || conv[j]) continue;
-      const double res = std::sqrt(nr[j]);
+      double res2 = 0.0;
+      for (int b = 0; b < rblk; ++b) res2 += nr[(size_t)b * nr_ + j];
+      const double res = std::sqrt(res2);
       rnorm[j] = res;
       if (res < cfg.tol_residual) {
         conv[j] = 1;
@@ -720,90 +1017,18 @@ static void davidson_run(qx_ctx* ctx, DavWork& W, int n, int ld, const double* d
       break;
     }
     if (newr.empty()) continue;
-    // Preconditioned residuals t_j (davidson.rs:444-449), staged after V.
     const int nnew = (int)newr.size();
-    for (int q = 0; q < nnew; ++q) {
-      const int j = newr[q];
-      double* t = W.V.p + (size_t)(nv + q) * ld;
-      QX_CUDA(cudaMemsetAsync(d_c, 0, sizeof(double), ctx->stream));
-      k_precond<<<1, kRedThreads, 0, ctx->stream>>>(W.R.p + (size_t)j * ld, d_delta, th[j], cfg.level_shift, n,
-                                                    t, d_c);
-      check_launch(ctx);
-      k_normalize<<<nblk, nthreads, 0, ctx->stream>>>(t, n, d_c, 1e-14);
-      check_launch(ctx);
-    }
     if (nv + nnew > max_space) {
       // Restart from the Ritz vectors, re-orthonormalised (davidson.rs:298-307).
-      QX_CUDA(cudaMemcpyAsync(W.V.p, W.X.p, (size_t)nr_ * ld * sizeof(double), cudaMemcpyDeviceToDevice,
-                              ctx->stream));
-      for (int i = 0; i < nr_; ++i) {
-        double* v = W.V.p + (size_t)i * ld;
-        for (int pass = 0; pass < 2 && i > 0; ++pass) {
-          GemmNT g{};
-          g.M = i;
-          g.N = 1;
-          g.K = n;
-          g.A = W.V.p;
-          g.lda = ld;
-          g.B = v;
-          g.ldb = ld;
-          g.C = d_c;
-          g.ldc = 1;
-          g.batch = 1;
-          g.alpha = 1.0;
-          g.splitk = 0;
-          gemm_nt_f64(ctx, g);
-          combine_rows(ctx, W.V.p, ld, i, d_c, 1, 1, n, v, ld, -1.0, 1.0);
-        }
-        QX_CUDA(cudaMemsetAsync(d_nrm, 0, sizeof(double), ctx->stream));
-        k_norm2<<<1, kRedThreads, 0, ctx->stream>>>(v, n, d_nrm);
-        check_launch(ctx);
-        k_normalize<<<nblk, nthreads, 0, ctx->stream>>>(v, n, d_nrm, -1.0);
-        check_launch(ctx);
-      }
+      std::vector<int> all_rows(nr_);
+      std::iota(all_rows.begin(), all_rows.end(), 0);
+      expand(0, W.X.p, all_rows, nullptr, th, -1.0);
       nv = nr_;
-      QX_CUDA(cudaMemsetAsync(W.V.p + (size_t)nv * ld, 0, (size_t)(cap - nv) * ld * sizeof(double), ctx->stream));
       apply(0, nv);
       continue;
     }
-    // Double Gram-Schmidt of each candidate against the subspace (davidson.rs:240-285).
-    int added = 0;
-    for (int q = 0; q < nnew; ++q) {
-      double* src = W.V.p + (size_t)(nv + q) * ld;
-      double* dst = W.V.p + (size_t)(nv + added) * ld;
-      if (src != dst)
-        QX_CUDA(cudaMemcpyAsync(dst, src, ld * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-      const int cur = nv + added;
-      for (int pass = 0; pass < 2; ++pass) {
-        GemmNT g{};
-        g.M = cur;
-        g.N = 1;
-        g.K = n;
-        g.A = W.V.p;
-        g.lda = ld;
-        g.B = dst;
-        g.ldb = ld;
-        g.C = d_c;
-        g.ldc = 1;
-        g.batch = 1;
-        g.alpha = 1.0;
-        g.splitk = 0;
-        gemm_nt_f64(ctx, g);
-        combine_rows(ctx, W.V.p, ld, cur, d_c, 1, 1, n, dst, ld, -1.0, 1.0);
-      }
-      QX_CUDA(cudaMemsetAsync(d_nrm, 0, sizeof(double), ctx->stream));
-      k_norm2<<<1, kRedThreads, 0, ctx->stream>>>(dst, n, d_nrm);
-      check_launch(ctx);
-      double h2 = 0.0;
-      QX_CUDA(cudaMemcpyAsync(&h2, d_nrm, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-      sync_and_check(ctx);
-      if (std::sqrt(h2) < cfg.lindep_threshold) continue;
-      k_normalize<<<nblk, nthreads, 0, ctx->stream>>>(dst, n, d_nrm, -1.0);
-      check_launch(ctx);
-      ++added;
-    }
-    QX_CUDA(cudaMemsetAsync(W.V.p + (size_t)(nv + added) * ld, 0, (size_t)(cap - nv - added) * ld * sizeof(double),
-                            ctx->stream));
+    // Preconditioned residuals (davidson.rs:444-449), each orthogonalised twice.
+    const int added = expand(nv, W.R.p, newr, d_delta, th, cfg.lindep_threshold);
     if (added > 0) apply(nv, added);
     nv += added;
   }
@@ -841,6 +1066,7 @@ qx_status qx_bse_davidson(qx_bse* B, const qx_davidson_config* cfgp, double* eig
                           int* converged_out, double* residual_norms, int* iterations) {
   if (!B || !cfgp) return QX_ERR_INVALID_INPUT;
   return bse_guard(B->ctx, [&] {
+    ensure_kd_f64(B);
     davidson_run(B->ctx, B->dav, B->nov, B->ldov, B->delta.p, B->h_delta,
                  [&](const double* x, double* y, int count) { bse_apply_rows(B, x, y, count); }, *cfgp, eigenvalues,
                  eigenvectors, converged_out, residual_norms, iterations);
