@@ -87,9 +87,10 @@ struct DigitArgs {
   const int2* xt;
   int wgroup;           // frequencies per group of the item order
   double* part;         // [2 n_tiles][nbatch][M]
-  // store: lower tiles and their mirror (lower = 1, with delta_mn added), or
-  // all; add: onto what out holds (a further range of K, no delta).
-  int lower, add;
+  // store: lower tiles and their mirror (lower = 1, with delta_mn added; add:
+  // onto what out holds, for a further range of K, no delta), or all tiles (wide:
+  // out and ldo allow 32-byte stores).
+  int lower, add, wide;
   double* out;
   int ldo;
   size_t out_stride;
@@ -143,8 +144,15 @@ __device__ __forceinline__ bool digit_tile(const DigitArgs& a, int it, int rank,
     }
     t.mb = t.nt + 2 * r + rank;
   } else {
-    t.nt = r % NT;
-    t.mb = r / NT * 2 + rank;
+    // The smaller operand stays in L2, the larger passes once.
+    const int mp = (T + 1) / 2;
+    if (a.N <= a.M) {
+      t.nt = r % NT;
+      t.mb = r / NT * 2 + rank;
+    } else {
+      t.nt = r / mp;
+      t.mb = (r - t.nt * mp) * 2 + rank;
+    }
   }
   t.kbe = kb;
   return true;
@@ -185,6 +193,24 @@ __device__ __forceinline__ double i64_to_f64(long long s) {
   const double hi = __hiloint2double(0x45300000, (int)(s >> 32) ^ 0x80000000);
   const double lo = __hiloint2double(0x43300000, (int)(uint32_t)s);
   return (hi - (0x1p84 + 0x1p63 + 0x1p52)) + lo;
+}
+
+// s 2^q, -1020 <= q <= 900, rounded to nearest even, without FP64 instructions
+// (the epilogue's get next to no issue slots while the MMAs run).
+__device__ __forceinline__ double i64_scale(long long s, int q) {
+  const unsigned long long sign = (unsigned long long)s & 0x8000000000000000ull;
+  const unsigned long long m = s < 0 ? 0ull - (unsigned long long)s : (unsigned long long)s;
+  if (m == 0) return 0.0;
+  const int lz = __clzll((long long)m);
+  const unsigned long long t = m << lz;
+  const uint32_t lo = (uint32_t)t;
+  const uint32_t up = (lo >> 10) & (uint32_t)(((lo & 0x3ff) != 0) | ((lo >> 11) & 1)) & 1;
+  const int e = 1022 + 63 - lz + q;  // the leading bit of t >> 11 adds one
+  return __longlong_as_double((long long)((((unsigned long long)(uint32_t)e << 52) + (t >> 11) + up) | sign));
+}
+
+__device__ __forceinline__ void st_v4(double* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
 }
 
 // A load that does not stay in L1.
@@ -326,6 +352,9 @@ __device__ __forceinline__ void digit_block_hi(DigitIssue& q, bool start, bool l
   q.publish(3, last);
 }
 
+// MODE: the epilogue (and args.rowdot, args.lower accordingly).
+enum { DIGIT_ROWDOT, DIGIT_LOWER, DIGIT_PLAIN };
+template <int MODE>
 __global__ void __launch_bounds__(dgt::THREADS, 1)
     k_digit_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, DigitArgs args) {
   namespace P = dgt;
@@ -521,7 +550,7 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
       constexpr int XB = 16;
       const int2* x = nullptr;
       int2 b[2][XB];
-      if (args.rowdot) {
+      if (MODE == DIGIT_ROWDOT) {
         x = args.xt + ((size_t)(t.mb * (P::TM / 32) + quarter) * args.ldsb + n0) * 32 + lane;
 #pragma unroll
         for (int q = 0; q < XB; ++q) b[0][q] = ld_stream(x + q * 32);
@@ -529,7 +558,7 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
       drain([&](int c, int d) { s[c] = ((s[c] + half_unit) >> args.sh) + ((long long)d << (40 - args.sh)); });
       if (!ok) break;
       const double sa = m < args.M ? args.scaleA[m] : 0.0;
-      if (args.rowdot) {
+      if (MODE == DIGIT_ROWDOT) {
         // Each thread contracts its row of C with its row of X, in integers:
         // FP64 instructions get next to no issue slots while the MMAs run at
         // full rate (with them this part of a tile took 16 000 to 36 000 cycles
@@ -573,22 +602,49 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
           v = emax == 2047 ? __longlong_as_double(0x7FF8000000000000ll) : ldexp(v * sa, emax - 1023 + args.sh - 28 - z) * sa;
           args.part[((size_t)(2 * t.nt + half) * args.nbatch + t.w) * args.M + m] = v;
         }
-      } else if (m < args.M) {
-        const double unit = sa * pow2i(args.sh - 40);  // C = s 2^(sh - 40), scaled
-        double* out = args.out + (size_t)t.w * args.out_stride;
-        double* orow = out + (size_t)m * args.ldo + n0;
+      } else if (MODE == DIGIT_LOWER) {
+        if (m < args.M) {
+          const double unit = sa * pow2i(args.sh - 40);  // C = s 2^(sh - 40), scaled
+          double* out = args.out + (size_t)t.w * args.out_stride;
+          double* orow = out + (size_t)m * args.ldo + n0;
 #pragma unroll
-        for (int c = 0; c < P::CPW; ++c) {
-          const int n = n0 + c;
-          if (n >= args.N || (args.lower && n > m)) continue;
-          double y = i64_to_f64(s[c]) * unit * __ldg(sb + c);
-          if (args.add)
-            y += orow[c];
-          else if (args.lower && n == m)
-            y += 1.0;
-          orow[c] = y;
-          // The lower triangle and its mirror: the stored matrix is exactly symmetric.
-          if (args.lower && n != m) out[(size_t)n * args.ldo + m] = y;
+          for (int c = 0; c < P::CPW; ++c) {
+            const int n = n0 + c;
+            if (n >= args.N || n > m) continue;
+            double y = i64_to_f64(s[c]) * unit * __ldg(sb + c);
+            if (args.add)
+              y += orow[c];
+            else if (n == m)
+              y += 1.0;
+            orow[c] = y;
+            // The lower triangle and its mirror: the stored matrix is exactly symmetric.
+            if (n != m) out[(size_t)n * args.ldo + m] = y;
+          }
+        }
+      } else if (m < args.M) {
+        // C = 2^(ea - 7) 2^(en - 7) 2^(sh - 40) s.  A tile of few K blocks is
+        // bound by this part: integer arithmetic and stores of whole 32-byte
+        // sectors where out allows them (16 800 x 5100 x 700: 2.0 ms with FP64
+        // instructions and 8-byte stores, now 1.26).  The scales are
+        // powers of two; one that is not a normal number (rows near the ends of
+        // the range, or not finite) takes the multiplication.
+        const int xs = (__double2hiint(sa) >> 20) & 2047;
+        const int xa = (xs == 0 || xs == 2047 ? 1 << 20 : xs) - 2046 + args.sh - 40;
+        const double unit = sa * pow2i(args.sh - 40);
+        double* orow = args.out + (size_t)t.w * args.out_stride + (size_t)m * args.ldo + n0;
+        auto value = [&](int c) {
+          const double sc = __ldg(sb + c);
+          const int xb = (__double2hiint(sc) >> 20) & 2047, q = xa + xb;
+          if (xb == 0 || xb == 2047 || q < -1020 || q > 900) return i64_to_f64(s[c]) * unit * sc;
+          return i64_scale(s[c], q);
+        };
+        if (args.wide && n0 + P::CPW <= args.N) {
+#pragma unroll
+          for (int c = 0; c < P::CPW; c += 4) st_v4(orow + c, value(c), value(c + 1), value(c + 2), value(c + 3));
+        } else {
+#pragma unroll
+          for (int c = 0; c < P::CPW; ++c)
+            if (n0 + c < args.N) orow[c] = value(c);
         }
       }
     }
@@ -850,7 +906,10 @@ static CUtensorMap digit_map(const int8_t* base, int K, int rows, int ldk, int s
   return m;
 }
 
+template <int MODE>
 static void launch_digit_gemm(qx_ctx* ctx, const int8_t* a, int lda, const int8_t* b, int ldb, DigitArgs args) {
+  args.rowdot = MODE == DIGIT_ROWDOT;
+  args.lower = MODE == DIGIT_LOWER;
   const CUtensorMap ma = digit_map(a, args.K, args.M, lda, dgt::NS, dgt::TM);
   const CUtensorMap mb = digit_map(b, args.K, args.N, ldb, dgt::NS * args.nbatch, dgt::TN / 2);
   QX_REQUIRE(args.K > 0 && args.K <= dgt::KMAX, QX_ERR_INVALID_INPUT, "digit GEMM: K = %d", args.K);
@@ -872,10 +931,10 @@ static void launch_digit_gemm(qx_ctx* ctx, const int8_t* a, int lda, const int8_
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   attr_once(ctx->device, [&] {
-    QX_CUDA(cudaFuncSetAttribute(k_digit_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, dgt::TOTAL));
+    QX_CUDA(cudaFuncSetAttribute(k_digit_gemm<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, dgt::TOTAL));
     cfg.gridDim = dim3(2 * ctx->sm_count);
     int n = 0;
-    QX_CUDA(cudaOccupancyMaxActiveClusters(&n, k_digit_gemm, &cfg));
+    QX_CUDA(cudaOccupancyMaxActiveClusters(&n, k_digit_gemm<MODE>, &cfg));
     max_clusters[ctx->device] = std::max(n, 1);
   });
   const int T = ceil_div(args.M, dgt::TM), NT = ceil_div(args.N, dgt::TN);
@@ -884,7 +943,7 @@ static void launch_digit_gemm(qx_ctx* ctx, const int8_t* a, int lda, const int8_
                   : (long long)(args.lower ? digit_lower_pairs(T) : ceil_div(T, 2) * NT) * args.nbatch;
   QX_REQUIRE(items > 0 && items < (1ll << 30), QX_ERR_INVALID_INPUT, "digit GEMM: %lld tiles", items);
   cfg.gridDim = dim3(2 * (unsigned)std::min<long long>(items, max_clusters[ctx->device]));
-  QX_CUDA(cudaLaunchKernelEx(&cfg, k_digit_gemm, ma, mb, args));
+  QX_CUDA(cudaLaunchKernelEx(&cfg, k_digit_gemm<MODE>, ma, mb, args));
   check_launch(ctx);
   ctx->pending.push_back({args.err, 1, 0});
 }
@@ -942,14 +1001,54 @@ bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int n
     a.scaleA = sa;
     a.scaleB = sb;
     a.ldsb = lds;
-    a.lower = 1;
     a.out = eps + (size_t)w0 * eps_stride;
     a.ldo = ldn;
     a.out_stride = eps_stride;
     for (int k0 = 0; k0 < nov; k0 += dgt::KMAX) {
       a.K = std::min(dgt::KMAX, nov - k0);
       a.add = k0 > 0;
-      launch_digit_gemm(ctx, da.as<int8_t>() + k0, ldk, db.as<int8_t>() + k0, ldk, a);
+      launch_digit_gemm<DIGIT_LOWER>(ctx, da.as<int8_t>() + k0, ldk, db.as<int8_t>() + k0, ldk, a);
+    }
+  }
+  return true;
+}
+
+// C[m][n] = sum_k A[m][k] B[n][k] (16-byte aligned rows, even lda and ldb).
+bool gemm_nt_digits(qx_ctx* ctx, const double* A, int M, int lda, const double* B, int N, int ldb, int K, double* C,
+                    int ldc) {
+  // From K = 161 on (two K blocks) and a few tiles each way: below, the
+  // padding and the digits cost what the faster products give.
+  if (K <= 160 || K > dgt::KMAX || M < 2 * dgt::TM || N < 2 * dgt::TN) return false;
+  const int ldd = round_up(K, 16);
+  const size_t row = (size_t)7 * ldd, budget = digit_budget(ctx);
+  const int cap = (int)std::min<size_t>(budget / row, 1u << 30) / 256 * 256;
+  const int mc = std::min(M, std::max(256, cap)), nc = std::min(N, std::max(256, cap));
+  const int lds = round_up(nc, dgt::TN);
+  DevBuf &da = ctx->ws[WS_DIG_A], &db = ctx->ws[WS_DIG_B], &ds = ctx->ws[WS_DIG_S];
+  if (!try_reserve(da, row * mc) || !try_reserve(db, row * nc) ||
+      !try_reserve(ds, ((size_t)mc + lds) * sizeof(double)))
+    return false;
+  double* sb = ds.as<double>();
+  double* sa = sb + lds;
+  QX_CUDA(cudaMemsetAsync(sb, 0, (size_t)lds * sizeof(double), ctx->stream));
+  for (int n0 = 0; n0 < N; n0 += nc) {
+    const int n = std::min(nc, N - n0);
+    split_rows(ctx, B + (size_t)n0 * ldb, n, K, ldb, 0, 1, 0, db.as<int8_t>(), ldd, sb, lds);
+    for (int m0 = 0; m0 < M; m0 += mc) {
+      const int m = std::min(mc, M - m0);
+      if (n0 == 0 || mc < M) split_rows(ctx, A + (size_t)m0 * lda, m, K, lda, 0, 1, 0, da.as<int8_t>(), ldd, sa, 0);
+      DigitArgs a{};
+      a.M = m;
+      a.N = n;
+      a.K = K;
+      a.nbatch = 1;
+      a.scaleA = sa;
+      a.scaleB = sb;
+      a.ldsb = lds;
+      a.out = C + (size_t)m0 * ldc + n0;
+      a.ldo = ldc;
+      a.wide = ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 31) == 0;
+      launch_digit_gemm<DIGIT_PLAIN>(ctx, da.as<int8_t>(), ldd, db.as<int8_t>(), ldd, a);
     }
   }
   return true;
@@ -989,7 +1088,6 @@ bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int np
       a.N = naux;
       a.K = naux;
       a.nbatch = n;
-      a.rowdot = 1;
       a.scaleA = sa;
       a.scaleB = sb;
       a.ldsb = lds;
@@ -997,7 +1095,7 @@ bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int np
       // Digits of W' of a frequency group within half of L2.
       a.wgroup = (int)std::max<size_t>(1, std::min<size_t>(n, ((size_t)60 << 20) / (row * naux)));
       a.part = dp.as<double>();
-      launch_digit_gemm(ctx, da.as<int8_t>(), ldd, db.as<int8_t>(), ldd, a);
+      launch_digit_gemm<DIGIT_ROWDOT>(ctx, da.as<int8_t>(), ldd, db.as<int8_t>(), ldd, a);
       k_digit_rowdot_sum<<<dim3(std::min(ceil_div(np, 256), 512), n), 256, 0, ctx->stream>>>(
           dp.as<double>(), 2 * NT, np, n, v + (size_t)w0 * ldv + p0, ldv);
       check_launch(ctx);

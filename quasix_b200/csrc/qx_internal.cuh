@@ -256,11 +256,14 @@ void launch_eps_fp64(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov
 bool chi_smooth(const double* energies, int nocc, int nvir, double wmax);
 
 // The FP64 contractions on the integer tensor pipe (k_digits.cu); false when
-// the device has no room for their operands (nothing was done).
+// the device has no room for their operands, or the product is too small for it
+// (nothing was done).
 bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw,
                        double* eps, int ldn, size_t eps_stride);
 bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc,
                                  int ldn, size_t wc_stride, int nw, double* v, int ldv);
+bool gemm_nt_digits(qx_ctx* ctx, const double* A, int M, int lda, const double* B, int N, int ldb, int K, double* C,
+                    int ldc);
 
 // ---------------------------------------------------------------------------
 // Guarded inversion (k_pivot.cu).  The block sweep has no pivoting; when eps

@@ -89,3 +89,17 @@ def test_non_finite_tensor_is_reported(q, bad):
     lpq[3, 5, 6] = lpq[3, 6, 5] = bad
     with pytest.raises(RuntimeError):
         q.get_sigma_diag(s.mo_energy, lpq, [5, 6], 6, nw=8)
+
+
+@pytest.mark.parametrize("nocc,nvir,naux", [(8, 31, 161), (8, 32, 161), (9, 43, 260)])
+def test_adjoint_at_tile_edges(q, nocc, nvir, naux):
+    """The adjoint's product over all frequencies (from naux 161 and dimension 256 on)."""
+    s = make_system(nocc, nvir, naux, seed=naux, pi_norm=2.0)
+    tg, nw = [nocc - 1, nocc], 9
+    vxc = np.diag(O.compute_exchange(np.ascontiguousarray(s.lpq[:, :, :nocc].transpose(1, 2, 0))))
+    r = q.g0w0_cd(s.mo_energy, s.lpq, nocc, tg, nw=nw, vxc=vxc, tol=1e-13, max_iter=100)
+    lam = np.array([1.0, 0.7])
+    ge, gl, _ = q.g0w0_cd_grad(s.mo_energy, s.lpq, nocc, tg, r["qp_energies"], lam, nw=nw)
+    oe, ol = O.g0w0_cd_grad(s.mo_energy, s.lpq, nocc, tg, r["qp_energies"], lam, nw)
+    assert np.abs(ge - oe).max() < 1e-10 * np.abs(oe).max()
+    assert np.abs(gl - ol).max() < 1e-10 * np.abs(ol).max()
