@@ -372,10 +372,11 @@ struct qx_bse {
   DevArr kd_split, kd_scale;
   int ldg = 0;
   bool kd = false;
-  // FP64: the contracted direct kernel C[(i,j)][(a,b)], formed by the first
-  // Davidson solve when it fits (ensure_kd_f64).
+  // FP64: the contracted direct kernel C[(i,j)][(a,b)], formed when it pays and
+  // fits (ensure_kd_f64), and the vectors applied so far.
   DevArr kd_f64;
   bool kd_f64_tried = false;
+  long long applied = 0;
   DevArr x_split;                    // split forms: hi/lo of the packed vectors
   DevArr xp, T, Yd, Z, Yx, Xr, Yr;  // matvec scratch
   DevArr gTt, gTp, gTpT, gdijT, gM, gG1, gG, gU;  // root-gradient scratch
@@ -385,40 +386,74 @@ struct qx_bse {
 };
 
 // Yd[i][a nvec + v] = sum_(j,b) C[(i,j)][(a,b)] X[v][(j,b)] for NV vectors from
-// v0 on.  What bounds it is reading C once (8 nov^2 bytes); each warp takes
-// KD_ROWS rows (i, a) of one i, its lanes along b, so that every C is used for
-// NV vectors and every X for KD_ROWS rows.
-constexpr int KD_ROWS = 2, KD_VECS = 6;
-template <int NV>
-__global__ void __launch_bounds__(128) k_kd_apply(const double* __restrict__ C, const double* __restrict__ X, int ldx,
-                                                  int nocc, int nvir, int nvec, int v0, double* __restrict__ Yd) {
+// v0 on.  What bounds it is reading C once (8 nov^2 bytes).  Each warp takes R
+// rows (i, a) of one i, its lanes along the (j, b) in one run (a run per j left
+// the last lanes of each idle), so that every C is used for NV vectors and every
+// X for R rows.  The next KD_LOADS entries of C are under way while a lane
+// multiplies the last ones.  865 MB for ten vectors: 404 us (612 us without the
+// prefetch, 426 us through a cp.async ring); 85 MB for five: 22 us.
+constexpr int KD_VECS = 10, KD_LOADS = 8;
+template <int R, int NV>
+__global__ void __launch_bounds__(128, R == 4 ? 3 : 4) k_kd_apply(const double* __restrict__ C,
+                                                                  const double* __restrict__ X, int ldx, int nocc,
+                                                                  int nvir, int nvec, int v0,
+                                                                  double* __restrict__ Yd) {
+  constexpr int U = KD_LOADS / R;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int i = blockIdx.y, a0 = (blockIdx.x * 4 + warp) * KD_ROWS;
+  const int i = blockIdx.y, a0 = (blockIdx.x * 4 + warp) * R;
   if (a0 >= nvir) return;
-  const int na = min(KD_ROWS, nvir - a0);
-  double acc[KD_ROWS][NV];
+  const int na = min(R, nvir - a0), nov = nocc * nvir;
+  double acc[R][NV];
 #pragma unroll
-  for (int a = 0; a < KD_ROWS; ++a)
+  for (int a = 0; a < R; ++a)
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[a][v] = 0.0;
-  for (int j = 0; j < nocc; ++j) {
-    const double* c = C + ((size_t)(i * nocc + j) * nvir + a0) * nvir;
-    const double* x = X + (size_t)v0 * ldx + (size_t)j * nvir;
-#pragma unroll 2
-    for (int b = lane; b < nvir; b += 32) {
+  const double* x = X + (size_t)v0 * ldx + lane;
+  // The lane's next entry of the run: f = j nvir + b, at c.
+  const double* c = C + ((size_t)i * nocc * nvir + a0) * nvir + lane;
+  const size_t skip = (size_t)(nvir - 1) * nvir;  // from b = nvir of j to b = 0 of j + 1
+  int b = lane, f = lane;
+  auto wrap = [&]() {
+    while (b >= nvir) {
+      b -= nvir;
+      c += skip;
+    }
+  };
+  wrap();
+  auto load = [&](double (&k)[R][U]) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int a = 0; a < R; ++a) k[a][u] = f < nov ? __ldcs(c + min(a, na - 1) * nvir) : 0.0;
+      f += 32;
+      b += 32;
+      c += 32;
+      wrap();
+    }
+  };
+  double k[R][U];
+  load(k);
+  for (int f0 = 0; f0 < nov; f0 += 32 * U) {
+    double next[R][U];
+    load(next);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = f0 + 32 * u + lane < nov;
       double xv[NV];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) xv[v] = __ldg(x + (size_t)v * ldx + b);
+      for (int v = 0; v < NV; ++v) xv[v] = in ? __ldg(x + (size_t)v * ldx + f0 + 32 * u) : 0.0;
 #pragma unroll
-      for (int a = 0; a < KD_ROWS; ++a) {
-        const double k = __ldg(c + (size_t)min(a, na - 1) * nvir + b);
+      for (int a = 0; a < R; ++a)
 #pragma unroll
-        for (int v = 0; v < NV; ++v) acc[a][v] = fma(k, xv[v], acc[a][v]);
-      }
+        for (int v = 0; v < NV; ++v) acc[a][v] = fma(k[a][u], xv[v], acc[a][v]);
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int a = 0; a < R; ++a) k[a][u] = next[a][u];
   }
 #pragma unroll
-  for (int a = 0; a < KD_ROWS; ++a)
+  for (int a = 0; a < R; ++a)
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       double s = acc[a][v];
@@ -427,73 +462,91 @@ __global__ void __launch_bounds__(128) k_kd_apply(const double* __restrict__ C, 
     }
 }
 
-static void kd_apply(qx_bse* B, const double* X, int nvec) {
-  qx_ctx* ctx = B->ctx;
-  const dim3 grid(ceil_div(ceil_div(B->nvir, KD_ROWS), 4), B->nocc);
-  for (int v0 = 0; v0 < nvec; v0 += KD_VECS) {
-    auto go = [&](auto nv) {
-      k_kd_apply<decltype(nv)::value><<<grid, 128, 0, ctx->stream>>>(B->kd_f64.p, X, B->ldov, B->nocc, B->nvir, nvec, v0,
-                                                                    B->Yd.p);
-    };
-    switch (std::min(KD_VECS, nvec - v0)) {
-      case 1: go(std::integral_constant<int, 1>()); break;
-      case 2: go(std::integral_constant<int, 2>()); break;
-      case 3: go(std::integral_constant<int, 3>()); break;
-      case 4: go(std::integral_constant<int, 4>()); break;
-      case 5: go(std::integral_constant<int, 5>()); break;
-      default: go(std::integral_constant<int, 6>()); break;
-    }
-    check_launch(ctx);
+template <int NV>
+static void launch_kd_apply(qx_bse* B, const double* X, int nv, int nvec, int v0) {
+  if constexpr (NV > 1) {
+    if (nv < NV) return launch_kd_apply<NV - 1>(B, X, nv, nvec, v0);
   }
+  qx_ctx* ctx = B->ctx;
+  auto go = [&](auto r) {
+    constexpr int R = decltype(r)::value;
+    k_kd_apply<R, NV><<<dim3(ceil_div(ceil_div(B->nvir, R), 4), B->nocc), 128, 0, ctx->stream>>>(
+        B->kd_f64.p, X, B->ldov, B->nocc, B->nvir, nvec, v0, B->Yd.p);
+  };
+  // Four rows per warp halve the reads of X through L1, which limit ten vectors
+  // with two; a small dimension needs the warps (12 per SM or more).
+  if ((long long)B->nocc * ceil_div(B->nvir, 4) >= 12ll * ctx->sm_count)
+    go(std::integral_constant<int, 4>());
+  else
+    go(std::integral_constant<int, 2>());
+  check_launch(ctx);
 }
 
-// FP64, before a Davidson solve: C[(i,j)][(a,b)] = sum_Q ijw[(i,j)][Q]
-// B_ab[(a,b)][Q] (kernel.rs:391-462 contracted once), batched over a from dabT.
-// A solve applies H a hundred times: the factored direct term costs 4 nov nvir
-// naux FLOPs per vector each time, C's one product 2 nov^2 naux FLOPs once.
-// (Dimension 3264, naux 560: 60 us against ~190 us per matvec of five vectors;
-// the product 0.8 ms.)  Held when its nov^2 doubles take at most 16 GB, the
-// bound of the split forms' K^d, and at most half of the free memory with the
-// product's operand; else, and below dimension 512, where both are a few
-// launches, the factored form stays.
-static void ensure_kd_f64(qx_bse* B) {
+static void kd_apply(qx_bse* B, const double* X, int nvec) {
+  const int passes = ceil_div(nvec, KD_VECS), per = ceil_div(nvec, passes);
+  for (int v0 = 0; v0 < nvec; v0 += per) launch_kd_apply<KD_VECS>(B, X, std::min(per, nvec - v0), nvec, v0);
+}
+
+// FP64: C[(i,j)][(a,b)] = sum_Q ijw[(i,j)][Q] B_ab[(a,b)][Q] (kernel.rs:391-462
+// contracted once).  The factored direct term costs 4 nov nvir naux FLOPs per
+// vector each time, C's one product 2 nov^2 naux FLOPs once, four times faster
+// as one product of digits: as much as nocc / 8 vectors with digits, nocc / 2
+// without.  It is formed when that many vectors have been applied the factored
+// way, so that no run of calls costs more than twice the better form; a solve of
+// n roots counts 8 n vectors ahead (it takes 10 to 100 per root).
+// Dimension 10 400, naux 1000, ten vectors: 3.1 ms factored, 0.6 ms contracted,
+// 2.5 ms to form it; dimension 3264, naux 560, five vectors: 190 and 60 us, 0.4 ms.
+// Held when its nov^2 doubles take at most 16 GB, the bound of the split forms'
+// K^d, and at most half of the free memory; else, and below dimension 512, where
+// both are a few launches, the factored form stays.
+static void ensure_kd_f64(qx_bse* B, long long vectors) {
   if (B->precision != QX_PREC_FP64 || B->kd_f64_tried) return;
+  if (vectors * (B->naux > 160 ? 8 : 2) < B->nocc) return;
   B->kd_f64_tried = true;
+  qx_ctx* ctx = B->ctx;
   const size_t n2 = (size_t)B->nov * B->nov;
   if (B->nov < 512 || n2 * sizeof(double) > ((size_t)16 << 30)) return;
-  qx_ctx* ctx = B->ctx;
-  DevArr dab;
-  const size_t dab_n = (size_t)B->nvir * B->nvir * B->ldq;
+  // dabT [a][Q][b] back to [a][b][Q], some virtuals a at a time.
+  const size_t slab = (size_t)B->nvir * B->ldq;
+  const int na = (int)std::max<size_t>(1, std::min<size_t>(B->nvir, ((size_t)64 << 20) / (slab * sizeof(double))));
   size_t avail = 0, total = 0;
   QX_CUDA(cudaMemGetInfo(&avail, &total));
-  if ((n2 + dab_n) * sizeof(double) > avail / 2) return;
+  if ((n2 + slab * na) * sizeof(double) > avail / 2) return;
+  DevArr dab;
   try {
     B->kd_f64.alloc(n2);
-    dab.alloc(dab_n);
+    dab.alloc(slab * na);
   } catch (const Error&) {
     cudaGetLastError();
     B->kd_f64.free();
     return;
   }
-  // dabT [a][Q][b] back to [a][b][Q].
-  QX_CUDA(cudaMemsetAsync(dab.p, 0, (size_t)B->nvir * B->nvir * B->ldq * sizeof(double), ctx->stream));
-  transpose(ctx, B->dabT.p, B->naux, B->nvir, B->ldvp, (size_t)B->naux * B->ldvp, dab.p, B->ldq,
-            (size_t)B->nvir * B->ldq, B->nvir);
-  GemmNT g{};
-  g.M = B->nocc * B->nocc;
-  g.N = B->nvir * B->nvir;
-  g.K = B->naux;
-  g.A = B->ijw.p;
-  g.lda = B->ldq;
-  g.B = dab.p;
-  g.ldb = B->ldq;
-  g.C = B->kd_f64.p;
-  g.ldc = B->nvir * B->nvir;
-  g.batch = 1;
-  g.alpha = 1.0;
-  g.splitk = 1;
-  gemm_nt_f64(ctx, g);
-  QX_CUDA(cudaStreamSynchronize(ctx->stream));  // dab is freed on return
+  try {
+    QX_CUDA(cudaMemsetAsync(dab.p, 0, slab * na * sizeof(double), ctx->stream));
+    for (int a0 = 0; a0 < B->nvir; a0 += na) {
+      const int n = std::min(na, B->nvir - a0);
+      transpose(ctx, B->dabT.p + (size_t)a0 * B->naux * B->ldvp, B->naux, B->nvir, B->ldvp, (size_t)B->naux * B->ldvp,
+                dab.p, B->ldq, slab, n);
+      GemmNT g{};
+      g.M = B->nocc * B->nocc;
+      g.N = n * B->nvir;
+      g.K = B->naux;
+      g.A = B->ijw.p;
+      g.lda = B->ldq;
+      g.B = dab.p;
+      g.ldb = B->ldq;
+      g.C = B->kd_f64.p + (size_t)a0 * B->nvir;
+      g.ldc = B->nvir * B->nvir;
+      g.batch = 1;
+      g.alpha = 1.0;
+      g.splitk = 1;
+      if (!gemm_nt_digits(ctx, g.A, g.M, g.lda, g.B, g.N, g.ldb, g.K, g.C, g.ldc)) gemm_nt_f64(ctx, g);
+    }
+    sync_and_check(ctx);  // dab is freed on return
+  } catch (...) {
+    B->kd_f64.free();
+    throw;
+  }
 }
 
 // y[v] = H x[v] for nvec vectors in row layout [nvec][ldov] (device).
@@ -502,6 +555,10 @@ static void ensure_kd_f64(qx_bse* B) {
 static void bse_apply_rows(qx_bse* B, const double* X, double* Y, int nvec, bool need_T = false) {
   qx_ctx* ctx = B->ctx;
   const int nocc = B->nocc, nvir = B->nvir, naux = B->naux;
+  if (!need_T) {
+    ensure_kd_f64(B, B->applied);
+    B->applied += nvec;
+  }
   B->Yd.alloc((size_t)nocc * nvir * nvec);
   if (B->kd_f64.p && !need_T) {
     kd_apply(B, X, nvec);
@@ -1066,7 +1123,7 @@ qx_status qx_bse_davidson(qx_bse* B, const qx_davidson_config* cfgp, double* eig
                           int* converged_out, double* residual_norms, int* iterations) {
   if (!B || !cfgp) return QX_ERR_INVALID_INPUT;
   return bse_guard(B->ctx, [&] {
-    ensure_kd_f64(B);
+    ensure_kd_f64(B, B->applied + 8ll * std::max(1, cfgp->n_roots));
     davidson_run(B->ctx, B->dav, B->nov, B->ldov, B->delta.p, B->h_delta,
                  [&](const double* x, double* y, int count) { bse_apply_rows(B, x, y, count); }, *cfgp, eigenvalues,
                  eigenvectors, converged_out, residual_norms, iterations);

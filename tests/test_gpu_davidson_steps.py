@@ -75,3 +75,26 @@ def test_contracted_direct_kernel(nocc, nvir, roots):
     assert np.abs(got["eigenvalues"] - np.linalg.eigvalsh(0.5 * (h + h.T))[:roots]).max() < 1e-9
     v = got["eigenvectors"]
     assert np.linalg.norm(h @ v - v * got["eigenvalues"], axis=0).max() < 2e-8
+
+
+@pytest.mark.parametrize("nocc,nvir,naux,nvec", [(17, 40, 170, 3), (17, 41, 161, 10), (16, 33, 260, 11), (8, 70, 90, 4),
+                                                 (15, 36, 200, 2), (20, 357, 48, 21)])
+def test_contracted_apply(nocc, nvir, naux, nvec):
+    """Blocks of vectors before and after the contracted direct kernel is formed
+    (with and without digits), against the factored oracle."""
+    import quasix_b200 as q
+    rng = np.random.default_rng(nvec)
+    dia, dij, dab = (rng.standard_normal(sh) * 0.05
+                     for sh in ((nocc * nvir, naux), (nocc * nocc, naux), (nvir * nvir, naux)))
+    w0 = np.eye(naux) + 0.01 * rng.standard_normal((naux, naux))
+    w0 = 0.5 * (w0 + w0.T)
+    delta = rng.uniform(0.3, 3.0, nocc * nvir)
+    k = q.BSETDAKernel(nocc, nvir, naux, delta, dia, dij, dab, w0)
+    x = rng.standard_normal((nocc * nvir, nvec))
+    ref = O.bse_apply_tda(x, delta, dia, dij, dab, w0, nocc, nvir)
+    for _ in range(4):  # factored at first, contracted when that has cost as much
+        got = k.apply_hamiltonian_batch(x)
+        assert np.abs(got - ref).max() < 1e-12 * np.abs(ref).max()
+    one = k.apply_hamiltonian_batch(np.ascontiguousarray(x[:, :1]))
+    k.close()
+    assert np.abs(one - ref[:, :1]).max() < 1e-12 * np.abs(ref).max()
