@@ -163,11 +163,6 @@ __device__ __forceinline__ void umma_i8_pair(uint32_t d, uint64_t a, uint64_t b,
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
       "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t p;
-  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
-  return p;
-}
 // kind::i8: signed 8-bit A and B (format 1), 32-bit integer accumulator
 // (format 2), both K-major, no saturation.
 constexpr uint32_t kDigitIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(dgt::TN >> 3) << 17) |

@@ -440,8 +440,11 @@ __global__ void __launch_bounds__(TcThreads<EPI, CONVB>::VALUE, 1)
       // epilogue sums the units in FP64, because the FP32 accumulation of the
       // tensor pipe carries a small same-signed error per step that grows
       // linearly over long positive sums (the diagonal of Pi over K = nov).
-      if (lane == 0) {
+      {
+        static_assert(TC_BK == 64, "descriptor words");
         const uint32_t idesc = umma_idesc_f16(TC_BM, BN, args.fp16);
+        const uint32_t elected = elect_one(), tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const uint32_t desc0 = umma_desc_lo(smem_u32(smem));
         int g = 0, u = 0;
         bool ok = true;
         for (int it = item0; it < n_items && ok; it += item_step) {
@@ -466,43 +469,40 @@ __global__ void __launch_bounds__(TcThreads<EPI, CONVB>::VALUE, 1)
             const bool unit_end = (EPI != EPI_ROWDOT) ? (kb % unit == unit - 1 || kb == kbe - 1) : kb == kbe - 1;
             const int buf = u % NBUF;
             if (unit_start && u >= NBUF) {
-              if (!mbar_wait(&acc_empty[buf], ((u / NBUF) - 1) & 1, abort_flag, args.err, 2)) {
-                ok = false;
-                break;
-              }
+              ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], ((u / NBUF) - 1) & 1, abort_flag, args.err, 2));
+              if (!ok) break;
             }
             const int s = g % TC_STAGES;
-            if (!mbar_wait(&full[s], (g / TC_STAGES) & 1, abort_flag, args.err, 3) ||
-                (CONVB && !mbar_wait(&conv[s], (g / TC_STAGES) & 1, abort_flag, args.err, 8))) {
-              ok = false;
-              break;
-            }
+            ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (g / TC_STAGES) & 1, abort_flag, args.err, 3) &&
+                                             (!CONVB || mbar_wait(&conv[s], (g / TC_STAGES) & 1, abort_flag, args.err, 8)));
+            if (!ok) break;
             tc_fence_after();
-            const uint32_t dacc = tmem_base + buf * BN;
-            uint8_t* st = smem + s * L::STAGE_BYTES;
-            const uint32_t ah = smem_u32(st), al = ah + L::A_BYTES;
-            const uint32_t bh = ah + 2 * L::A_BYTES, bl = bh + L::B_BYTES;
+            const uint32_t dacc = tmem + buf * BN;
+            const uint32_t ah = desc0 + s * (L::STAGE_BYTES >> 4), al = ah + (L::A_BYTES >> 4);
+            const uint32_t bh = ah + (2 * L::A_BYTES >> 4), bl = bh + (L::B_BYTES >> 4);
+            if (elected) {
 #pragma unroll
-            for (int kk = 0; kk < TC_BK / 16; ++kk) {
-              const uint32_t off = kk * 32;
-              const uint32_t acc0 = (!unit_start || kk > 0) ? 1u : 0u;
-              umma_f16(dacc, umma_desc<TC_BK>(ah + off), umma_desc<TC_BK>(bh + off), idesc, acc0);
-              umma_f16(dacc, umma_desc<TC_BK>(ah + off), umma_desc<TC_BK>(bl + off), idesc, 1u);
-              umma_f16(dacc, umma_desc<TC_BK>(al + off), umma_desc<TC_BK>(bh + off), idesc, 1u);
+              for (int kk = 0; kk < TC_BK / 16; ++kk) {
+                const uint32_t acc0 = (!unit_start || kk > 0) ? 1u : 0u;
+                umma_f16(dacc, umma_desc_of(ah + 2 * kk), umma_desc_of(bh + 2 * kk), idesc, acc0);
+                umma_f16(dacc, umma_desc_of(ah + 2 * kk), umma_desc_of(bl + 2 * kk), idesc, 1u);
+                umma_f16(dacc, umma_desc_of(al + 2 * kk), umma_desc_of(bh + 2 * kk), idesc, 1u);
+              }
+              umma_commit(&empty[s]);
+              if (unit_end) umma_commit(&acc_full[buf]);
             }
-            umma_commit(&empty[s]);
-            if (unit_end) {
-              umma_commit(&acc_full[buf]);
-              ++u;
-            }
+            __syncwarp();
+            if (unit_end) ++u;
           }
         }
         }
         // Wait until every MMA this thread issued has completed (TMEM and the
         // stages are released only after that).
-        umma_commit(drain);
-        volatile int no_abort = 0;
-        mbar_wait(drain, 0, &no_abort, args.err, 6);
+        if (elected) {
+          umma_commit(drain);
+          volatile int no_abort = 0;
+          mbar_wait(drain, 0, &no_abort, args.err, 6);
+        }
       }
     } else if (CONVB && warp >= 2 + TcWarps<EPI>::NEPI) {
       // ---------------- B operand converters (CONVB) ----------------
@@ -1573,8 +1573,10 @@ __global__ void __launch_bounds__(pairrd::THREADS, 1)
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (even CTA) ----------------
-    if (leader && lane == 0) {
+    if (leader) {
       const uint32_t idesc = umma_idesc_f16(2 * TC_BM, P::BN, args.fp16);
+      const uint32_t elected = elect_one(), tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+      const uint32_t desc0 = umma_desc_lo(smem_u32(smem));
       int gk = 0, t = 0;
       bool ok = true;
       for (int it = item0; it < n_items && ok; it += item_step) {
@@ -1585,37 +1587,38 @@ __global__ void __launch_bounds__(pairrd::THREADS, 1)
         for (int nt = 0; nt < n_tiles && ok; ++nt, ++t) {
           const int kbe = kbe_of(nt);
           const int buf = t & 1;
-          if (t >= 2 && !mbar_wait(&acc_empty[buf], ((t / 2) - 1) & 1, abort_flag, args.err, 33)) {
-            ok = false;
-            break;
-          }
-          const uint32_t dacc = tmem_base + buf * P::BN;
+          ok = __all_sync(0xffffffffu, t < 2 || mbar_wait(&acc_empty[buf], ((t / 2) - 1) & 1, abort_flag, args.err, 33));
+          if (!ok) break;
+          const uint32_t dacc = tmem + buf * P::BN;
           for (int kb = 0; kb < kbe; ++kb, ++gk) {
             const int s = gk % P::STAGES;
-            if (!mbar_wait(&full[s], (gk / P::STAGES) & 1, abort_flag, args.err, 34)) {
-              ok = false;
-              break;
-            }
+            ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (gk / P::STAGES) & 1, abort_flag, args.err, 34));
+            if (!ok) break;
             tc_fence_after();
-            const uint32_t ah = smem_u32(smem + s * P::STAGE_BYTES), al = ah + P::A_BYTES;
-            const uint32_t bh = ah + 2 * P::A_BYTES, bl = bh + P::B_BYTES;
+            const uint32_t ah = desc0 + s * (P::STAGE_BYTES >> 4), al = ah + (P::A_BYTES >> 4);
+            const uint32_t bh = ah + (2 * P::A_BYTES >> 4), bl = bh + (P::B_BYTES >> 4);
+            if (elected) {
 #pragma unroll
-            for (int kk = 0; kk < P::BK / 16; ++kk) {
-              const uint32_t off = kk * 32;
-              const uint32_t acc0 = (kb > 0 || kk > 0) ? 1u : 0u;
-              umma_f16_pair(dacc, umma_desc<P::BK>(ah + off), umma_desc<P::BK>(bh + off), idesc, acc0);
-              umma_f16_pair(dacc, umma_desc<P::BK>(ah + off), umma_desc<P::BK>(bl + off), idesc, 1u);
-              umma_f16_pair(dacc, umma_desc<P::BK>(al + off), umma_desc<P::BK>(bh + off), idesc, 1u);
+              for (int kk = 0; kk < P::BK / 16; ++kk) {
+                const uint32_t acc0 = (kb > 0 || kk > 0) ? 1u : 0u;
+                umma_f16_pair(dacc, umma_desc_of(ah + 2 * kk), umma_desc_of(bh + 2 * kk), idesc, acc0);
+                umma_f16_pair(dacc, umma_desc_of(ah + 2 * kk), umma_desc_of(bl + 2 * kk), idesc, 1u);
+                umma_f16_pair(dacc, umma_desc_of(al + 2 * kk), umma_desc_of(bh + 2 * kk), idesc, 1u);
+              }
+              umma_commit_pair_both(&empty[s]);
             }
-            umma_commit_pair_both(&empty[s]);
+            __syncwarp();
           }
           if (!ok) break;
-          umma_commit_pair_both(&acc_full[buf]);
+          if (elected) umma_commit_pair_both(&acc_full[buf]);
+          __syncwarp();
         }
       }
-      umma_commit_pair_own(drain);
-      volatile int no_abort = 0;
-      mbar_wait(drain, 0, &no_abort, args.err, 35);
+      if (elected) {
+        umma_commit_pair_own(drain);
+        volatile int no_abort = 0;
+        mbar_wait(drain, 0, &no_abort, args.err, 35);
+      }
     }
   } else {
     // ---------------- epilogue (warps 2..9, both CTAs): row dot products ----------------
@@ -1961,8 +1964,10 @@ __global__ void __launch_bounds__(pairp0::THREADS, 1)
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (even CTA) ----------------
-    if (leader && lane == 0) {
+    if (leader) {
       const uint32_t idesc = umma_idesc_f16(2 * TC_BM, TC_BM, args.fp16);
+      const uint32_t elected = elect_one(), tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+      const uint32_t desc0 = umma_desc_lo(smem_u32(smem));
       int g = 0, u = 0;
       bool ok = true;
       for (int it = item0; it < n_items && ok; it += item_step) {
@@ -1970,38 +1975,38 @@ __global__ void __launch_bounds__(pairp0::THREADS, 1)
           const bool unit_start = kb % unit == 0;
           const bool unit_end = kb % unit == unit - 1 || kb == k_blocks - 1;
           const int buf = u % P::NBUF;
-          if (unit_start && u >= P::NBUF &&
-              !mbar_wait(&acc_empty[buf], ((u / P::NBUF) - 1) & 1, abort_flag, args.err, 23)) {
-            ok = false;
-            break;
+          if (unit_start && u >= P::NBUF) {
+            ok = __all_sync(0xffffffffu,
+                            mbar_wait(&acc_empty[buf], ((u / P::NBUF) - 1) & 1, abort_flag, args.err, 23));
+            if (!ok) break;
           }
           const int s = g % P::STAGES;
-          if (!mbar_wait(&full[s], (g / P::STAGES) & 1, abort_flag, args.err, 24)) {
-            ok = false;
-            break;
-          }
+          ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (g / P::STAGES) & 1, abort_flag, args.err, 24));
+          if (!ok) break;
           tc_fence_after();
-          const uint32_t dacc = tmem_base + buf * TC_BM;
-          const uint32_t ah = smem_u32(smem + s * P::STAGE_BYTES), al = ah + P::A_BYTES;
-          const uint32_t bh = ah + 2 * P::A_BYTES, bl = bh + P::B_BYTES;
+          const uint32_t dacc = tmem + buf * TC_BM;
+          const uint32_t ah = desc0 + s * (P::STAGE_BYTES >> 4), al = ah + (P::A_BYTES >> 4);
+          const uint32_t bh = ah + (2 * P::A_BYTES >> 4), bl = bh + (P::B_BYTES >> 4);
+          if (elected) {
 #pragma unroll
-          for (int kk = 0; kk < P::BK / 16; ++kk) {
-            const uint32_t off = kk * 32;
-            const uint32_t acc0 = (!unit_start || kk > 0) ? 1u : 0u;
-            umma_f16_pair(dacc, umma_desc<P::BK>(ah + off), umma_desc<P::BK>(bh + off), idesc, acc0);
-            umma_f16_pair(dacc, umma_desc<P::BK>(ah + off), umma_desc<P::BK>(bl + off), idesc, 1u);
-            umma_f16_pair(dacc, umma_desc<P::BK>(al + off), umma_desc<P::BK>(bh + off), idesc, 1u);
+            for (int kk = 0; kk < P::BK / 16; ++kk) {
+              const uint32_t acc0 = (!unit_start || kk > 0) ? 1u : 0u;
+              umma_f16_pair(dacc, umma_desc_of(ah + 2 * kk), umma_desc_of(bh + 2 * kk), idesc, acc0);
+              umma_f16_pair(dacc, umma_desc_of(ah + 2 * kk), umma_desc_of(bl + 2 * kk), idesc, 1u);
+              umma_f16_pair(dacc, umma_desc_of(al + 2 * kk), umma_desc_of(bh + 2 * kk), idesc, 1u);
+            }
+            umma_commit_pair_both(&empty[s]);
+            if (unit_end) umma_commit_pair_both(&acc_full[buf]);
           }
-          umma_commit_pair_both(&empty[s]);
-          if (unit_end) {
-            umma_commit_pair_both(&acc_full[buf]);
-            ++u;
-          }
+          __syncwarp();
+          if (unit_end) ++u;
         }
       }
-      umma_commit_pair_own(drain);
-      volatile int no_abort = 0;
-      mbar_wait(drain, 0, &no_abort, args.err, 25);
+      if (elected) {
+        umma_commit_pair_own(drain);
+        volatile int no_abort = 0;
+        mbar_wait(drain, 0, &no_abort, args.err, 25);
+      }
     }
   } else {
     // ---------------- epilogue (warps 2..9, both CTAs) ----------------

@@ -90,6 +90,23 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
 }
 
 
+// An issuer of MMAs runs its loop in all 32 lanes, with the same values, and one
+// elected lane issues: the descriptors then stay in uniform registers.  With the
+// whole loop inside one lane's branch every MMA waited for its descriptors to be
+// moved there, ~105 cycles per MMA against the 64 that M x N x K = 128 x 128 x 16
+// (256 x 128 x 16 of a pair) occupies the tensor core.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p;
+}
+// Descriptor of the operand at saddr in two words, K blocks of 64 elements
+// (umma_desc<64>): 16 elements of K advance the low word by 2.
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFF) >> 4) | (1u << 16); }
+__device__ __forceinline__ uint64_t umma_desc_of(uint32_t lo) {
+  return ((uint64_t)(64u | (1u << 14) | (2u << 29)) << 32) | lo;
+}
+
 // Instruction descriptor: kind::f16 with bf16 (fmt 1) or fp16 (fmt 0) A and B of
 // the same type, f32 accumulator, K-major A and B.
 __host__ __device__ constexpr uint32_t umma_idesc_f16(int M, int N, int fp16) {
