@@ -11,7 +11,9 @@
 
 namespace qx {
 
-using GemmTile = F64Tile<64, 64, 2, 2, 3>;
+// Eight warps of 16 x 32: the products of a Davidson step 22.0 -> 18.7 us each
+// against four of 32 x 32.
+using GemmTile = F64Tile<64, 64, 4, 2, 3>;
 
 // C[b][m][n] (or the split-K partial) = sum_{k in split} A[b][m][k] B[b][n][k]
 __global__ void __launch_bounds__(GemmTile::THREADS) k_gemm_nt(GemmNT g, double* __restrict__ part) {

@@ -43,7 +43,9 @@ void launch_chi(qx_ctx* ctx, const double* energies, int nocc, int nvir, const d
 // eps[w] = I + B_ov diag(chi'[w]) B_ov^T on lower-triangular tile pairs,
 // mirrored on store.
 // ---------------------------------------------------------------------------
-using EpsTile = F64Tile<64, 64, 2, 2, 3>;
+// Eight warps of 16 x 32 (four of 32 x 32 left the FP64 tensor pipe waiting on
+// its operands: 22.5 us at naux 139 / nov 352, now 18.1; a batch 658 -> 572 us).
+using EpsTile = F64Tile<64, 64, 4, 2, 3>;
 
 __global__ void __launch_bounds__(EpsTile::THREADS) k_eps_f64(const double* __restrict__ bov, int ldov, int naux,
                                                               int nov, const double* __restrict__ chi,
@@ -330,7 +332,9 @@ __global__ void __launch_bounds__(512) k_sweep_diag(const double* __restrict__ M
                          growth ? growth + w : nullptr);
 }
 
-using PanelTile = F64Tile<64, 64, 2, 2, 3>;
+// Two stages: K is 128, and five blocks fit an SM instead of three (32 matrices
+// of order 1000: 455 -> 341 us).
+using PanelTile = F64Tile<64, 64, 2, 2, 2>;
 
 // *out = max(*out, max over the block of m) (m >= 0 compares as its bit
 // pattern); every thread of the block calls it; red holds one double per warp.
@@ -396,7 +400,10 @@ __global__ void __launch_bounds__(PanelTile::THREADS) k_sweep_tpanel(const doubl
                     amax ? amax + w : nullptr);
 }
 
-using SweepTile = F64Tile<64, 64, 2, 2, 3>;
+// Eight warps and two stages: 40 warps per SM hide the read-modify-write of the
+// tile (four warps and three stages: 2.08 ms for the updates of 32 matrices of
+// order 1000, four and two 1.55, now 1.48; 128 x 128 tiles 2.5 to 2.9).
+using SweepTile = F64Tile<64, 64, 4, 2, 2>;
 
 // M[r][c] -= T[r] . P[c] over the 64 x 64 tile (tm, tn), lower part; rows and
 // columns of the K block are left alone.  mode 0: any tile; 1: only tiles whose
@@ -1242,10 +1249,13 @@ void launch_exchange_diag(qx_ctx* ctx, const double* lpq, int naux, int nmo, int
 // ---------------------------------------------------------------------------
 // Pair contraction: v[w][p] = 2 sum_Q Bpt[p][Q] sum_{P <= Q} W'[w][Q][P] Bpt[p][P]
 // with W' the half-lower form of Wc (k_finish_wc), i.e. Bpt[p]^T Wc[w] Bpt[p].
-// One CTA per (128-pair block, frequency); it walks every Q tile, so the
+// One CTA per (64-pair block, frequency); it walks every Q tile, so the
 // per-pair sums stay in shared memory and are written once (deterministic).
 // ---------------------------------------------------------------------------
-using PairTile = F64Tile<128, 64, 4, 2, 3>;
+// 64 pairs per block: the contractions that come here (naux up to 160, or no
+// room for digits) leave SMs idle with 128 (23.5 and 44.5 us at nmo 24 and 40,
+// now 14.3 and 26.8).
+using PairTile = F64Tile<64, 64, 4, 2, 3>;
 
 __global__ void __launch_bounds__(PairTile::THREADS) k_pair_contract_f64(const double* __restrict__ bpt, int ldk,
                                                                          int npair, int naux,
