@@ -146,7 +146,8 @@ __global__ void __launch_bounds__(256) k_ritz(const double* __restrict__ V, cons
 // barrier after each set of partial dot products (two per candidate), which
 // every block then adds in the same order.  STAGE: the block's columns of V are
 // kept in shared memory for the launch, so that between the barriers nothing
-// but the partial dots comes from L2.  (As separate GEMM, combination and
+// but the partial dots comes from L2; else they are read from L2 four times per
+// candidate, by 32 warps instead of eight.  (As separate GEMM, combination and
 // norm launches with a host decision per candidate, a step of five candidates
 // took 40 launches and five synchronisations: ~450 us at n = 3264, now 87 us.)
 constexpr int kExpandMax = 64, kExpandRed = 128, kExpandSmem = 220 * 1024;
@@ -156,25 +157,27 @@ struct DavExpand {
   const double* src;
   const double* delta;
   double shift, lindep;
+  int t_smem;    // unstaged: the candidate is in shared memory
   double* part;  // [2][gridDim.x][cap + 1]
   int* added;
   int idx[kExpandMax];
   double theta[kExpandMax];
 };
 template <bool STAGE>
-__global__ void __launch_bounds__(256) k_dav_expand(DavExpand a) {
+__global__ void __launch_bounds__(STAGE ? 256 : 1024) k_dav_expand(DavExpand a) {
+  constexpr int NW = STAGE ? 8 : 32;
   extern __shared__ double sm[];
   const int G = gridDim.x, g = blockIdx.x;
   const int L = (a.n + G - 1) / G, x0 = g * L, len = max(0, min(L, a.n - x0)), ldc = a.cap + 1;
-  double* red = sm;           // [8][kExpandRed]
-  double* c = red + 8 * kExpandRed;  // [cap + 1] summed dot products
-  double* vs = c + ldc;       // [cap][L] staged rows
+  double* red = sm;                   // [NW][kExpandRed]
+  double* c = red + NW * kExpandRed;  // [cap + 1] summed dot products
+  double* vs = c + ldc;               // [cap][L] staged rows
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   cooperative_groups::grid_group grid = cooperative_groups::this_grid();
   const size_t ps = (size_t)G * ldc;
   int cur = a.nv + *a.added;
   // The candidate's columns of this block.
-  double* t = STAGE ? vs + a.cap * L : a.V + (size_t)cur * a.ld + x0;
+  double* t = STAGE ? vs + a.cap * L : a.t_smem ? vs : a.V + (size_t)cur * a.ld + x0;
   if (STAGE)
     for (int i = warp; i < cur; i += 8)
       for (int x = lane; x < len; x += 32) vs[i * L + x] = a.V[(size_t)i * a.ld + x0 + x];
@@ -182,9 +185,10 @@ __global__ void __launch_bounds__(256) k_dav_expand(DavExpand a) {
   // Dots of t with rows 0 .. cur (row cur: t itself) -> c, through part[b].
   auto dots = [&](int b) {
     double* out = a.part + b * ps + (size_t)g * ldc;
-    for (int i = warp; i <= cur; i += 8) {
+    for (int i = warp; i <= cur; i += NW) {
       double s = 0.0;
       const double* v = i < cur ? row(i) : t;
+#pragma unroll 4
       for (int x = lane; x < len; x += 32) s += v[x] * t[x];
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (lane == 0) out[i] = s;
@@ -197,14 +201,14 @@ __global__ void __launch_bounds__(256) k_dav_expand(DavExpand a) {
       for (int i = lane; i < m; i += 32) {
         double s = 0.0;
 #pragma unroll 8
-        for (int q = warp; q < G; q += 8) s += __ldcg(in + (size_t)q * ldc + i0 + i);
+        for (int q = warp; q < G; q += NW) s += __ldcg(in + (size_t)q * ldc + i0 + i);
         red[warp * kExpandRed + i] = s;
       }
       __syncthreads();
       if (tid < m) {
         double s = 0.0;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) s += red[w * kExpandRed + tid];
+        for (int w = 0; w < NW; ++w) s += red[w * kExpandRed + tid];
         c[i0 + tid] = s;
       }
       __syncthreads();
@@ -212,6 +216,28 @@ __global__ void __launch_bounds__(256) k_dav_expand(DavExpand a) {
   };
   // t = f t - f sum_i c[i] V[i]
   auto subtract = [&](double f) {
+    if (!STAGE) {
+      // Warps over chunks of 32 columns and, where there are fewer chunks than
+      // warps, over groups of rows.
+      const int nxb = (L + 31) / 32, cpb = min(nxb, NW), groups = NW / cpb;
+      for (int c0 = 0; c0 < nxb; c0 += cpb) {
+        const int x = 32 * (c0 + warp % cpb) + lane, rg = warp / cpb;
+        double s = 0.0;
+        if (rg < groups && x < len) {
+#pragma unroll 8
+          for (int i = rg; i < cur; i += groups) s += c[i] * a.V[(size_t)i * a.ld + x0 + x];
+        }
+        red[warp * 32 + lane] = s;
+        __syncthreads();
+        if (warp < cpb && x < len) {
+          double u = 0.0;
+          for (int q = 0; q < groups; ++q) u += red[(q * cpb + warp) * 32 + lane];
+          t[x] = f * (t[x] - u);
+        }
+        __syncthreads();
+      }
+      return;
+    }
     for (int xb = 0; xb < len; xb += 32) {
       const int x = xb + lane;
       double s = 0.0;
@@ -233,7 +259,7 @@ __global__ void __launch_bounds__(256) k_dav_expand(DavExpand a) {
   grid.sync();  // every block has read *added
   for (int q = 0; q < a.count; ++q) {
     const double* r = a.src + (size_t)a.idx[q] * a.ld + x0;
-    for (int x = tid; x < len; x += 256) {
+    for (int x = tid; x < len; x += 32 * NW) {
       double v = r[x];
       if (a.delta) {
         double den = a.delta[x0 + x] - a.theta[q] + a.shift;
@@ -256,14 +282,14 @@ __global__ void __launch_bounds__(256) k_dav_expand(DavExpand a) {
     subtract(1.0);
     if (h < a.lindep) continue;
     const double inv = 1.0 / h;
-    for (int x = tid; x < len; x += 256) {
+    for (int x = tid; x < len; x += 32 * NW) {
       const double v = t[x] * inv;
       a.V[(size_t)cur * a.ld + x0 + x] = v;
       if (STAGE) vs[cur * L + x] = v;
     }
     __syncthreads();
     ++cur;
-    if (!STAGE) t += a.ld;
+    if (!STAGE && !a.t_smem) t += a.ld;
   }
   if (g == 0 && tid == 0) *a.added = cur - a.nv;
 }
@@ -958,10 +984,11 @@ static void davidson_run(qx_ctx* ctx, DavWork& W, int n, int ld, const double* d
   };
   // (Staged rows up to the limit of shared memory; beyond, V and the candidate
   // stay in global memory.)
-  const size_t expand_base = ((size_t)8 * kExpandRed + cap + 1) * sizeof(double);
-  const size_t expand_rows = (size_t)(cap + 1) * ceil_div(n, xblk) * sizeof(double);
-  const bool stage = expand_base + expand_rows <= (size_t)kExpandSmem;
-  const size_t expand_smem = expand_base + (stage ? expand_rows : 0);
+  const size_t expand_row = (size_t)ceil_div(n, xblk) * sizeof(double);
+  const auto expand_base = [&](int nw) { return ((size_t)nw * kExpandRed + cap + 1) * sizeof(double); };
+  const bool stage = expand_base(8) + (cap + 1) * expand_row <= (size_t)kExpandSmem;
+  const bool t_smem = stage || expand_base(32) + expand_row <= (size_t)kExpandSmem;
+  const size_t expand_smem = stage ? expand_base(8) + (cap + 1) * expand_row : expand_base(32) + (t_smem ? expand_row : 0);
   static PerDeviceOnce attr_once;
   attr_once(ctx->device, [&] {
     QX_CUDA(cudaFuncSetAttribute(k_dav_expand<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kExpandSmem));
@@ -985,13 +1012,14 @@ static void davidson_run(qx_ctx* ctx, DavWork& W, int n, int ld, const double* d
       a.shift = cfg.level_shift;
       a.lindep = lindep;
       a.part = W.part.p;
+      a.t_smem = t_smem;
       a.added = d_added;
       for (int q = 0; q < a.count; ++q) {
         a.idx[q] = list[q0 + q];
         a.theta[q] = delta ? theta[list[q0 + q]] : 0.0;
       }
       void* args[] = {&a};
-      QX_CUDA(cudaLaunchCooperativeKernel(stage ? (const void*)k_dav_expand<true> : (const void*)k_dav_expand<false>, dim3(xblk), dim3(256), args, expand_smem,
+      QX_CUDA(cudaLaunchCooperativeKernel(stage ? (const void*)k_dav_expand<true> : (const void*)k_dav_expand<false>, dim3(xblk), dim3(stage ? 256 : 1024), args, expand_smem,
                                           ctx->stream));
       check_launch(ctx);
     }
