@@ -717,8 +717,9 @@ def main():
     if prec_main == "fp64":
         dpeak = fp64_dgemm_peak_tflops()
         roof = {"bound": "tensor", "achieved": achieved, "peak": dpeak, "unit": "TFLOP/s", "frac": achieved / dpeak,
-                "traffic": None, "kernel": "k_pair_contract_f64",
-                "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64 has no entry in MEASURED_PEAKS.json)"}
+                "traffic": None, "kernel": "k_digit_gemm",
+                "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64 has no entry in MEASURED_PEAKS.json); "
+                               "the kernel forms its products on the integer tensor pipe and can exceed it"}
     else:
         pk = peaks.get("bf16_tflops_sustained", peaks.get("bf16_tflops"))
         cform = "single" if args.contraction_form == "single" else "pair"

@@ -114,10 +114,12 @@ void launch_eps_fp64(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov
 // no pivot vanishes).  Per block of SWEEP_NB columns:
 //   k_sweep_diag   : D = inverse of the current diagonal block (one CTA per matrix)
 //   k_sweep_tpanel : T = M[:, K] D                      (DMMA GEMM, K = nb)
-//   k_sweep_write  : P[r] = M[r][K] (old panel), then M[r][K] = M[K][r] = T[r],
+//   k_sweep_write  : P[r] = M[r][K] (old panel), then M[r][K] or M[K][r] = T[r],
 //                    M[K][K] = -D
 //   k_sweep_update : M[r][c] -= T[r] . P[c]  for r, c outside K, lower tiles
-//                    only, mirrored (DMMA GEMM, K = nb)
+//                    only (DMMA GEMM, K = nb)
+// M lives in the lower triangle, with the next block's rows mirrored; a guarded
+// sweep keeps both triangles.
 // Because the update reads the saved panel P, the next block's diagonal and
 // panel can be swept while the rest of this block's update still runs: the
 // update is split into the tiles that touch the next block (on the critical

@@ -1831,8 +1831,10 @@ __global__ void k_chi_cols(const double* __restrict__ chi, int nov, int ldov, co
 // the FP64 sums of the single-CTA epilogue the pair took 2.35 ms, its MMAs
 // waiting on the drain of the accumulators; with the compensated FP32 sums
 // 1.74 ms, against 1.69 ms for single-CTA tiles (which drain in FP64: the
-// compensated sums measured no faster there).  The single-CTA form stays the
-// default; this one is QX_P0_PAIR.
+// compensated sums measured no faster there).  Since the MMAs are issued from
+// warp-uniform code the GEMM alone takes 1.11 ms, against 1.23 ms for
+// single-CTA tiles.  The single-CTA form stays the default, for its FP64 sums;
+// this one is QX_P0_PAIR.
 namespace pairp0 {
 constexpr int STAGES = 4;
 constexpr int BK = 64;
@@ -2325,8 +2327,8 @@ SweepSplit launch_sweep_split(qx_ctx* ctx, cudaStream_t st, const double* Tp, co
 }
 
 // M[w][r][c] -= sum_q T[w][r][q] P[w][c][q] on stream st over the lower
-// 128 x 128 tiles outside tile row/column kblk (the K block), mirrored;
-// mode / next_blk select the look-ahead subset (filter_mode of TcArgs).  err
+// 128 x 128 tiles outside tile row/column kblk (the K block), the next block's
+// rows mirrored; mode / next_blk select the look-ahead subset (filter_mode of TcArgs).  err
 // is one status word, zero on entry.
 void launch_sweep_update_tc(qx_ctx* ctx, cudaStream_t st, double* eps, int n, int ldn, size_t stride, int nw,
                             int kblk, const SweepSplit& sp, int mode, int next_blk, int* err) {
