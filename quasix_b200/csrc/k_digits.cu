@@ -39,6 +39,7 @@
 // issued while the MMAs run at full rate.
 #include <algorithm>
 
+#include "digit_rowdot.cuh"
 #include "qx_internal.cuh"
 #include "tc_ptx.cuh"
 
@@ -559,17 +560,14 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
         // full rate (with them this part of a tile took 16 000 to 36 000 cycles
         // and ended only when the next tile's low pass had, its high pass
         // waiting).  The row of s is shifted up until its largest entry takes
-        // 63 bits; the columns' scales enter as shifts below the largest of
-        // them; of each product 2^4 X s the part above 2^64 is kept (|X| <
+        // 62 bits; the columns' scales enter as shifts below the largest of
+        // them; of each product 2^5 X s the part above 2^64 is kept (|X| <
         // 2^55, so 16 of them fit 62 bits).  X is laid out so that a load is 256
         // contiguous bytes per warp.
         uint32_t top = 0;
 #pragma unroll
-        for (int c = 0; c < P::CPW; ++c) {
-          const int h = (int)(s[c] >> 32);
-          top |= (uint32_t)(h ^ (h >> 31));
-        }
-        const int z = __clz(top) - 1;
+        for (int c = 0; c < P::CPW; ++c) top |= rowdot::top_bits(s[c]);
+        const int z = rowdot::norm_shift(top);
         // Exponent fields of the columns' scales (2047: a row that is not finite).
         const int emax = __reduce_max_sync(0xffffffffu, max(__double2hiint(__ldg(sb + lane)) >> 20,
                                                             __double2hiint(__ldg(sb + lane + 32)) >> 20));
@@ -586,15 +584,13 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
           for (int q = 0; q < XB; ++q) {
             const int dn = min(emax - (__double2hiint(__ldg(sb + c0 + q)) >> 20), 63);
             const long long y = (s[c0 + q] << z) >> dn;
-            const int yl = (int)(uint32_t)y, yh = (int)(y >> 32) - (yl >> 31);  // y = 2^32 yh + yl, yl signed
-            acc += (long long)b[h][q].y * yh;
-            acc += __mulhi(b[h][q].y, yl) + __mulhi(b[h][q].x, yh);
+            acc += rowdot::term(b[h][q].x, b[h][q].y, y);
           }
           v += i64_to_f64(acc);
         }
         if (m < args.M) {
           // b = 2^(ea - 55) X, C = 2^(ea - 7) 2^(en - 7) 2^(sh - 40) s.
-          v = emax == 2047 ? __longlong_as_double(0x7FF8000000000000ll) : ldexp(v * sa, emax - 1023 + args.sh - 28 - z) * sa;
+          v = emax == 2047 ? __longlong_as_double(0x7FF8000000000000ll) : ldexp(v * sa, emax - 1023 + args.sh - (24 + rowdot::XSHIFT) - z) * sa;
           args.part[((size_t)(2 * t.nt + half) * args.nbatch + t.w) * args.M + m] = v;
         }
       } else if (MODE == DIGIT_LOWER) {
@@ -792,7 +788,7 @@ __global__ void __launch_bounds__(256) k_digit_split(const double* __restrict__ 
 }
 
 // Rows of b [rows][ld] (K valid columns, scales sa as left by k_digit_split)
-// as the integers that their digits stand for, times 2^4: xt[r / 32][k][r % 32]
+// as the integers that their digits stand for, times 2^XSHIFT: xt[r / 32][k][r % 32]
 // = {signed low word, high word}, k < ldt, zero outside.  Blocks of 32 rows x 32
 // columns through shared memory.
 __global__ void __launch_bounds__(256) k_digit_xt(const double* __restrict__ b, int rows, int K, int ld,
@@ -810,9 +806,8 @@ __global__ void __launch_bounds__(256) k_digit_xt(const double* __restrict__ b, 
   int2* dst = xt + ((size_t)blockIdx.y * ldt + k0) * 32;
   for (int y = threadIdx.x >> 5; y < 32; y += 8) {
     const double v = tile[tx][y];
-    const long long X = fin ? __double2ll_rn(v * f1 * f2) << 4 : 0;
-    const int lo = (int)(uint32_t)X;
-    dst[y * 32 + tx] = make_int2(lo, (int)(X >> 32) - (lo >> 31));
+    const rowdot::Words w = rowdot::words(fin ? __double2ll_rn(v * f1 * f2) << rowdot::XSHIFT : 0);
+    dst[y * 32 + tx] = make_int2(w.lo, w.hi);
   }
 }
 
