@@ -1,6 +1,6 @@
 // Integer arithmetic of the digit kernel's row-dot epilogue (k_digits.cu):
-// acc += the part of X y above 2^64, in units of 2^64, from 32-bit words.
-// Plain C++ apart from the two intrinsics, so that it can be run on the host.
+// sums of products of a 56-bit and a 63-bit integer from 32-bit words.
+// Plain C++ apart from one intrinsic, so that it can be run on the host.
 #pragma once
 #include <stdint.h>
 
@@ -15,21 +15,25 @@ namespace rowdot {
 
 #ifdef __CUDA_ARCH__
 QX_HD int clz32(uint32_t x) { return __clz((int)x); }
-QX_HD int mulhi32(int a, int b) { return __mulhi(a, b); }
 #else
 QX_HD int clz32(uint32_t x) { return x ? __builtin_clz(x) : 32; }
-QX_HD int mulhi32(int a, int b) { return (int)(((int64_t)a * b) >> 32); }
 #endif
 
-// The integers of b times 2^XSHIFT: |X| < 2^60.
-constexpr int XSHIFT = 5;
-
-// v = 2^32 hi + lo, lo signed.  hi takes a carry when bit 31 of v is set: |v|
-// < 2^63 - 2^31, or it would wrap.
+// X = 2^28 hi + lo, |X| < 0.996 2^55: |lo| <= 2^27, |hi| < 0.997 2^27.
+constexpr int XBITS = 28;
 struct Words {
   int lo, hi;
 };
-QX_HD Words words(int64_t v) {
+QX_HD Words x_words(int64_t v) {
+  Words w;
+  w.lo = (int)((uint32_t)v << (32 - XBITS)) >> (32 - XBITS);
+  w.hi = (int)((v - w.lo) >> XBITS);
+  return w;
+}
+
+// y = 2^32 hi + lo, lo signed.  hi takes a carry when bit 31 of y is set: |y|
+// < 2^63 - 2^31, or it would wrap.
+QX_HD Words y_words(int64_t v) {
   Words w;
   w.lo = (int)(uint32_t)v;
   w.hi = (int)((uint32_t)(int32_t)(v >> 32) - (uint32_t)(w.lo >> 31));
@@ -47,11 +51,26 @@ QX_HD uint32_t top_bits(int64_t s) {
 // with the wrong sign.)
 QX_HD int norm_shift(uint32_t top) { return clz32(top) - 2; }
 
-// |X| < 2^60 and |y| < 2^62, so that the sum of 16 terms stays below 2^62 + 2^35.
-QX_HD int64_t term(int xlo, int xhi, int64_t y) {
-  const Words w = words(y);
-  return (int64_t)xhi * w.hi + mulhi32(xhi, w.lo) + mulhi32(xlo, w.hi);
-}
+// The sum of TERMS products X y, |y| <= 2^62, in units of 2^60, without the
+// product of the low words: |hi hi| <= 2^57, |hi lo| <= 2^58, |lo hi| <= 2^57,
+// and TERMS of each stay below 2^63.  The middle sums join as a whole, rounded
+// to nearest: floors of each product added up to an error of one sign, 32 units
+// per 16 terms at most.
+constexpr int TERMS = 16, UNIT = 60;
+struct Sum {
+  int64_t hh = 0, hl = 0, lh = 0;
+  QX_HD void add(int xlo, int xhi, int64_t y) {
+    const Words w = y_words(y);
+    hh += (int64_t)xhi * w.hi;
+    hl += (int64_t)xhi * w.lo;
+    lh += (int64_t)xlo * w.hi;
+  }
+  template <int B>
+  QX_HD static int64_t rounded(int64_t m) {
+    return (m >> B) + ((m >> (B - 1)) & 1);
+  }
+  QX_HD int64_t result() const { return hh + rounded<32>(hl) + rounded<XBITS>(lh); }
+};
 
 }  // namespace rowdot
 }  // namespace qx

@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
       drain([&](int c, int d) { s[c] += (long long)d << 32; });
       // With D_0, in units of 2^(sh + 8) so that the sum stays below 2^63.
       const long long half_unit = args.sh ? 1ll << (args.sh - 1) : 0;
-      constexpr int XB = 16;
+      constexpr int XB = rowdot::TERMS;
       const int2* x = nullptr;
       int2 b[2][XB];
       if (MODE == DIGIT_ROWDOT) {
@@ -561,9 +561,8 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
         // and ended only when the next tile's low pass had, its high pass
         // waiting).  The row of s is shifted up until its largest entry takes
         // 62 bits; the columns' scales enter as shifts below the largest of
-        // them; of each product 2^5 X s the part above 2^64 is kept (|X| <
-        // 2^55, so 16 of them fit 62 bits).  X is laid out so that a load is 256
-        // contiguous bytes per warp.
+        // them; of each product X s the part above 2^60 is kept.  X is laid out so
+        // that a load is 256 contiguous bytes per warp.
         uint32_t top = 0;
 #pragma unroll
         for (int c = 0; c < P::CPW; ++c) top |= rowdot::top_bits(s[c]);
@@ -579,18 +578,19 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
 #pragma unroll
             for (int q = 0; q < XB; ++q) b[h ^ 1][q] = ld_stream(x + (c0 + XB + q) * 32);
           }
-          long long acc = 0;
+          rowdot::Sum acc;
 #pragma unroll
           for (int q = 0; q < XB; ++q) {
             const int dn = min(emax - (__double2hiint(__ldg(sb + c0 + q)) >> 20), 63);
             const long long y = (s[c0 + q] << z) >> dn;
-            acc += rowdot::term(b[h][q].x, b[h][q].y, y);
+            acc.add(b[h][q].x, b[h][q].y, y);
           }
-          v += i64_to_f64(acc);
+          v += i64_to_f64(acc.result());
         }
         if (m < args.M) {
           // b = 2^(ea - 55) X, C = 2^(ea - 7) 2^(en - 7) 2^(sh - 40) s.
-          v = emax == 2047 ? __longlong_as_double(0x7FF8000000000000ll) : ldexp(v * sa, emax - 1023 + args.sh - (24 + rowdot::XSHIFT) - z) * sa;
+          v = emax == 2047 ? __longlong_as_double(0x7FF8000000000000ll)
+                           : ldexp(v * sa, emax - 1023 + args.sh - (88 - rowdot::UNIT) - z) * sa;
           args.part[((size_t)(2 * t.nt + half) * args.nbatch + t.w) * args.M + m] = v;
         }
       } else if (MODE == DIGIT_LOWER) {
@@ -788,8 +788,8 @@ __global__ void __launch_bounds__(256) k_digit_split(const double* __restrict__ 
 }
 
 // Rows of b [rows][ld] (K valid columns, scales sa as left by k_digit_split)
-// as the integers that their digits stand for, times 2^XSHIFT: xt[r / 32][k][r % 32]
-// = {signed low word, high word}, k < ldt, zero outside.  Blocks of 32 rows x 32
+// as the integers that their digits stand for: xt[r / 32][k][r % 32] = {low word,
+// high word} (rowdot::x_words), k < ldt, zero outside.  Blocks of 32 rows x 32
 // columns through shared memory.
 __global__ void __launch_bounds__(256) k_digit_xt(const double* __restrict__ b, int rows, int K, int ld,
                                                   const double* __restrict__ sa, int ldt, int2* __restrict__ xt) {
@@ -806,7 +806,7 @@ __global__ void __launch_bounds__(256) k_digit_xt(const double* __restrict__ b, 
   int2* dst = xt + ((size_t)blockIdx.y * ldt + k0) * 32;
   for (int y = threadIdx.x >> 5; y < 32; y += 8) {
     const double v = tile[tx][y];
-    const rowdot::Words w = rowdot::words(fin ? __double2ll_rn(v * f1 * f2) << rowdot::XSHIFT : 0);
+    const rowdot::Words w = rowdot::x_words(fin ? __double2ll_rn(v * f1 * f2) : 0);
     dst[y * 32 + tx] = make_int2(w.lo, w.hi);
   }
 }

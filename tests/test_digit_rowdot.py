@@ -2,9 +2,8 @@
 the host from its source against exact Python integers.
 
 A row of 64 sums s (|s| < 2^62) is normalised to 62 bits and multiplied with
-the integers X of a pair (|X| < 2^55 before their shift); the part of each
-product above 2^64 is kept.  Per term that drops less than two units (the floors
-of the two middle products) and a quarter (low x low).
+the integers X of a pair (|X| < 2^55); the part of each product above 2^60 is kept.  A term's low x low product drops less than a quarter
+of a unit, the sum of 16 rounds twice.
 """
 import ctypes
 import os
@@ -18,22 +17,21 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 HARNESS = """
 #include "digit_rowdot.cuh"
 using namespace qx::rowdot;
-// Sum over 64 columns in units of 2^64, and the shift of the row.
+// Sum over 64 columns in units of 2^60, and the shift of the row.
 extern "C" int rowdot64(const int64_t* s, const int64_t* X, int64_t* out) {
   uint32_t top = 0;
   for (int c = 0; c < 64; ++c) top |= top_bits(s[c]);
   const int z = norm_shift(top);
-  for (int c0 = 0; c0 < 64; c0 += 16) {
-    int64_t acc = 0;
-    for (int q = c0; q < c0 + 16; ++q) {
-      const Words x = words(X[q] << XSHIFT);
-      acc += term(x.lo, x.hi, s[q] << z);
+  for (int c0 = 0; c0 < 64; c0 += TERMS) {
+    Sum acc;
+    for (int q = c0; q < c0 + TERMS; ++q) {
+      const Words x = x_words(X[q]);
+      acc.add(x.lo, x.hi, s[q] << z);
     }
-    out[c0 / 16] = acc;
+    out[c0 / TERMS] = acc.result();
   }
   return z;
 }
-extern "C" int xshift() { return XSHIFT; }
 """
 
 
@@ -64,23 +62,43 @@ def _edges():
 @pytest.mark.parametrize("xtop", [2 ** 54 - 1, int(0.995 * 2 ** 55), -int(0.995 * 2 ** 55), 3])
 def test_largest_sums_keep_their_sign(lib, xtop):
     rng = np.random.default_rng(0)
-    xs = lib.xshift()
     for lead in _edges():
         s = rng.integers(-abs(lead) // 8 - 1, abs(lead) // 8 + 1, 64)
         X = rng.integers(-2 ** 53, 2 ** 53, 64)
         s[17], X[17] = lead, xtop
         got, z = _rowdot(lib, s, X)
-        exact = sum((int(x) << xs) * (int(y) << z) for x, y in zip(X, s))
-        assert abs(got * 2 ** 64 - exact) <= 64 * 2.25 * 2 ** 64, (lead, z)
+        exact = sum(int(x) * (int(y) << z) for x, y in zip(X, s))
+        assert abs(got * 2 ** 60 - exact) <= 64 * (0.25 + 2 * 0.5 / 16) * 2 ** 60, (lead, z)
 
 
 def test_sums_of_sixteen_fit(lib):
     """Every term at its largest, all of one sign."""
-    xs = lib.xshift()
     for sx in (1, -1):
         for lead in (2 ** 62 - 1, 2 ** 61, 2 ** 62 - 2 ** 30):
             s = np.full(64, lead)
             X = np.full(64, sx * int(0.996 * 2 ** 55))
             got, z = _rowdot(lib, s, X)
-            exact = sum((int(x) << xs) * (int(y) << z) for x, y in zip(X, s))
-            assert abs(got * 2 ** 64 - exact) <= 64 * 2.25 * 2 ** 64
+            exact = sum(int(x) * (int(y) << z) for x, y in zip(X, s))
+            assert abs(got * 2 ** 60 - exact) <= 64 * (0.25 + 2 * 0.5 / 16) * 2 ** 60
+
+
+def test_error_has_no_sign(lib):
+    """4000 random rows: eight roundings of each, variance 1 / 12, and 64 low
+    products of variance 1 / 144; the mean error stays within six of its
+    standard deviations."""
+    rng = np.random.default_rng(1)
+    err = []
+    for _ in range(4000):
+        s = rng.integers(-2 ** 61, 2 ** 61, 64)
+        X = rng.integers(-2 ** 54, 2 ** 54, 64)
+        got, z = _rowdot(lib, s, X)
+        exact = sum(int(x) * (int(y) << z) for x, y in zip(X, s))
+        err.append((got * 2 ** 60 - exact) / 2 ** 60)
+    sd = np.sqrt(8 / 12 + 64 / 144)
+    assert np.std(err) < 1.1 * sd
+    assert abs(np.mean(err)) < 6 * sd / np.sqrt(len(err))
+
+
+def test_zero_rows(lib):
+    assert _rowdot(lib, np.zeros(64), np.full(64, 5))[0] == 0
+    assert _rowdot(lib, np.full(64, 5), np.zeros(64))[0] == 0
