@@ -14,9 +14,9 @@ namespace qx {
 namespace rowdot {
 
 #ifdef __CUDA_ARCH__
-QX_HD int clz32(uint32_t x) { return __clz((int)x); }
+QX_HD int clz64(uint64_t x) { return __clzll((int64_t)x); }
 #else
-QX_HD int clz32(uint32_t x) { return x ? __builtin_clz(x) : 32; }
+QX_HD int clz64(uint64_t x) { return x ? __builtin_clzll(x) : 64; }
 #endif
 
 // X = 2^28 hi + lo, |X| < 0.996 2^55: |lo| <= 2^27, |hi| < 0.997 2^27.
@@ -40,16 +40,30 @@ QX_HD Words y_words(int64_t v) {
   return w;
 }
 
-// The bits of |s| >> 32 (ones' complement), for the OR over a row.
-QX_HD uint32_t top_bits(int64_t s) {
-  const int h = (int)(s >> 32);
-  return (uint32_t)(h ^ (h >> 31));
+// The sums of a row stand in units of their columns' scales; dn (0 .. 63) is how
+// far a column's scale lies below the largest of the 64.  The row is
+// normalised in the units of that largest scale; where no column lies further
+// below than NEAR, by the sums as they are (dn 0), which costs NEAR bits at most.
+constexpr int NEAR = 3;
+
+// The bits of |s| in these units (ones' complement), for the OR over a row.
+QX_HD uint64_t top_bits(int64_t s, int dn) {
+  const int64_t h = s >> dn;
+  return (uint64_t)(h ^ (h >> 63));
 }
 
 // Shift by which a row's sums (|s| < 2^62) take 62 bits: one bit is left for the
 // carry into the high word.  (With 63 bits a sum within 2^31 of 2^63 came out
 // with the wrong sign.)
-QX_HD int norm_shift(uint32_t top) { return clz32(top) - 2; }
+QX_HD int norm_shift(uint64_t top) { return clz64(top) - 2; }
+
+// The sum shifted up by z in these units.  (With the shift taken from the sums
+// as they are, a column of small scale and large sum left the others, and itself
+// after its own shift down, that many bits fewer.)
+QX_HD int64_t aligned(int64_t s, int z, int dn) {
+  const int up = z - dn;
+  return up >= 0 ? (int64_t)((uint64_t)s << up) : s >> -up;
+}
 
 // The sum of TERMS products X y, |y| <= 2^62, in units of 2^60, without the
 // product of the low words: |hi hi| <= 2^57, |hi lo| <= 2^58, |lo hi| <= 2^57,

@@ -559,33 +559,58 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
         // FP64 instructions get next to no issue slots while the MMAs run at
         // full rate (with them this part of a tile took 16 000 to 36 000 cycles
         // and ended only when the next tile's low pass had, its high pass
-        // waiting).  The row of s is shifted up until its largest entry takes
-        // 62 bits; the columns' scales enter as shifts below the largest of
-        // them; of each product X s the part above 2^60 is kept.  X is laid out so
-        // that a load is 256 contiguous bytes per warp.
-        uint32_t top = 0;
+        // waiting).  The row of s is shifted up until its largest entry takes 62
+        // bits in units of the largest of the columns' scales; of each product X s
+        // the part above 2^60 is kept.  X is laid out so that a load is 256
+        // contiguous bytes per warp.
+        // Exponent fields of the columns' scales (2047: a row that is not finite; 0:
+        // a zero row or none), and how far each lies below the largest: column
+        // 32 j + l in lane l.
+        int dn[P::CPW / 32], emax = 0, spread = 0;
 #pragma unroll
-        for (int c = 0; c < P::CPW; ++c) top |= rowdot::top_bits(s[c]);
-        const int z = rowdot::norm_shift(top);
-        // Exponent fields of the columns' scales (2047: a row that is not finite).
-        const int emax = __reduce_max_sync(0xffffffffu, max(__double2hiint(__ldg(sb + lane)) >> 20,
-                                                            __double2hiint(__ldg(sb + lane + 32)) >> 20));
+        for (int j = 0; j < P::CPW / 32; ++j) emax = max(emax, dn[j] = __double2hiint(__ldg(sb + 32 * j + lane)) >> 20);
+        emax = __reduce_max_sync(0xffffffffu, emax);
+#pragma unroll
+        for (int j = 0; j < P::CPW / 32; ++j) {
+          if (dn[j]) spread = max(spread, emax - dn[j]);
+          dn[j] = min(emax - dn[j], 63);
+        }
+        spread = __reduce_max_sync(0xffffffffu, spread);
+        int z;
         double v = 0.0;
+        auto contract = [&](auto&& y) {
 #pragma unroll
-        for (int c0 = 0; c0 < P::CPW; c0 += XB) {
-          const int h = (c0 / XB) & 1;
-          if (c0 + XB < P::CPW) {
+          for (int c0 = 0; c0 < P::CPW; c0 += XB) {
+            const int h = (c0 / XB) & 1;
+            if (c0 + XB < P::CPW) {
 #pragma unroll
-            for (int q = 0; q < XB; ++q) b[h ^ 1][q] = ld_stream(x + (c0 + XB + q) * 32);
+              for (int q = 0; q < XB; ++q) b[h ^ 1][q] = ld_stream(x + (c0 + XB + q) * 32);
+            }
+            rowdot::Sum acc;
+#pragma unroll
+            for (int q = 0; q < XB; ++q) acc.add(b[h][q].x, b[h][q].y, y(c0 + q));
+            v += i64_to_f64(acc.result());
           }
-          rowdot::Sum acc;
+        };
+        // Scales within 2^3 of each other, as those of a dielectric matrix's rows:
+        // the shift is taken from the sums as they are, which costs three bits at
+        // most.  (The other form for all tiles took 1 to 3 % longer for the whole
+        // call, nmo 121 to 300.)
+        uint64_t top = 0;
 #pragma unroll
-          for (int q = 0; q < XB; ++q) {
-            const int dn = min(emax - (__double2hiint(__ldg(sb + c0 + q)) >> 20), 63);
-            const long long y = (s[c0 + q] << z) >> dn;
-            acc.add(b[h][q].x, b[h][q].y, y);
-          }
-          v += i64_to_f64(acc.result());
+        for (int c = 0; c < P::CPW; ++c) top |= rowdot::top_bits(s[c], 0);
+        z = rowdot::norm_shift(top);
+        if (__all_sync(0xffffffffu, spread <= rowdot::NEAR && z >= rowdot::NEAR)) {
+          contract([&](int c) {  // (a zero column's shift does not matter)
+            return (long long)((unsigned long long)s[c] << ((z - emax + (__double2hiint(__ldg(sb + c)) >> 20)) & 63));
+          });
+        } else {
+          auto down = [&](int c) { return __shfl_sync(0xffffffffu, dn[c / 32], c % 32); };
+          top = 0;
+#pragma unroll
+          for (int c = 0; c < P::CPW; ++c) top |= rowdot::top_bits(s[c], down(c));
+          z = rowdot::norm_shift(top);
+          contract([&](int c) { return rowdot::aligned(s[c], z, down(c)); });
         }
         if (m < args.M) {
           // b = 2^(ea - 55) X, C = 2^(ea - 7) 2^(en - 7) 2^(sh - 40) s.
@@ -667,7 +692,8 @@ __global__ void k_digit_rowdot_sum(const double* __restrict__ part, int np, int 
 // f1 * f2 = 2^(55 - e) lie within the digits' range (the margin for the
 // balanced top digit: below 0x7F7F7F7F7F7F80 = 0.996 * 2^55), sc = 2^(e - 7).
 // A row with an infinity or a NaN gets zero digits and a NaN scale: what it
-// enters becomes NaN.
+// enters becomes NaN.  A zero row gets the scale zero, so that it does not stand
+// for the largest scale among rows of small entries.
 struct RowScale {
   double f1, f2, sc;
 };
@@ -678,7 +704,12 @@ __device__ __forceinline__ RowScale digit_scale(unsigned long long amax) {
     r.sc = __longlong_as_double(0x7FF8000000000000ll);
     return r;
   }
-  int e = amax == 0 ? 0 : max(1, (int)(amax >> 52)) - 1022;
+  if (amax == 0) {
+    r.f1 = r.f2 = 1.0;
+    r.sc = 0.0;
+    return r;
+  }
+  int e = max(1, (int)(amax >> 52)) - 1022;
   if ((amax & 0xFFFFFFFFFFFFFull) >= 0xFC00000000000ull) ++e;
   const int k = 55 - e, k1 = k >> 1;
   r.f1 = pow2i(k1);
@@ -798,9 +829,10 @@ __global__ void __launch_bounds__(256) k_digit_xt(const double* __restrict__ b, 
   for (int y = threadIdx.x >> 5; y < 32; y += 8)
     tile[y][tx] = (r0 + y < rows && k0 + tx < K) ? b[(size_t)(r0 + y) * ld + k0 + tx] : 0.0;
   __syncthreads();
-  // 2^(55 - e) in two factors, from the scale 2^(e - 7); zero for a row that is not finite.
-  const double sc = r0 + tx < rows ? sa[r0 + tx] : 1.0;
-  const bool fin = isfinite(sc);
+  // 2^(55 - e) in two factors, from the scale 2^(e - 7); zero for a row that is
+  // not finite or zero.
+  const double sc = r0 + tx < rows ? sa[r0 + tx] : 0.0;
+  const bool fin = sc > 0.0 && isfinite(sc);
   const int k = 48 - (fin ? ilogb(sc) : 0), k1 = k >> 1;
   const double f1 = fin ? pow2i(k1) : 0.0, f2 = pow2i(k - k1);
   int2* dst = xt + ((size_t)blockIdx.y * ldt + k0) * 32;
