@@ -38,6 +38,7 @@
 // in registers (64 per thread), as integers: FP64 instructions hardly get
 // issued while the MMAs run at full rate.
 #include <algorithm>
+#include <cmath>
 
 #include "digit_rowdot.cuh"
 #include "qx_internal.cuh"
@@ -594,19 +595,19 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
         };
         // Scales within 2^3 of each other, as those of a dielectric matrix's rows:
         // the shift is taken from the sums as they are, which costs three bits at
-        // most.  (The other form for all tiles took 1 to 3 % longer for the whole
-        // call, nmo 121 to 300.)
-        uint64_t top = 0;
+        // most, and from their high words.  (The other form for all tiles took 1 to
+        // 3 % longer for the whole call, nmo 121 to 300.)
+        uint32_t high = 0;
 #pragma unroll
-        for (int c = 0; c < P::CPW; ++c) top |= rowdot::top_bits(s[c], 0);
-        z = rowdot::norm_shift(top);
-        if (__all_sync(0xffffffffu, spread <= rowdot::NEAR && z >= rowdot::NEAR)) {
+        for (int c = 0; c < P::CPW; ++c) high |= (uint32_t)(rowdot::top_bits(s[c], 0) >> 32);
+        z = rowdot::norm_shift((uint64_t)high << 32);
+        if (__all_sync(0xffffffffu, spread <= rowdot::NEAR && z >= rowdot::NEAR && (high != 0 || m >= args.M || emax == 0))) {
           contract([&](int c) {  // (a zero column's shift does not matter)
             return (long long)((unsigned long long)s[c] << ((z - emax + (__double2hiint(__ldg(sb + c)) >> 20)) & 63));
           });
         } else {
           auto down = [&](int c) { return __shfl_sync(0xffffffffu, dn[c / 32], c % 32); };
-          top = 0;
+          uint64_t top = 0;
 #pragma unroll
           for (int c = 0; c < P::CPW; ++c) top |= rowdot::top_bits(s[c], down(c));
           z = rowdot::norm_shift(top);
@@ -674,14 +675,54 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
   }
 }
 
-// v[w][p] = 2 sum_q part[q][w][p]  (fixed order)
-__global__ void k_digit_rowdot_sum(const double* __restrict__ part, int np, int npair, int nw,
-                                   double* __restrict__ v, int ldv) {
-  const int w = blockIdx.y;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npair; p += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int q = 0; q < np; ++q) s += part[((size_t)q * nw + w) * npair + p];
-    v[(size_t)w * ldv + p] = 2.0 * s;
+// v[w][p] = 2 sum_q part[q][w][p]  (fixed order), and the items (w, block of
+// REDO_ROWS pairs) whose digits may not hold v as the DMMA kernel would: list[0 ..
+// *count), in any order.
+//
+// Fixed point loses what an entry lacks of its row's bound, so the error of v is
+// not bounded by v's own terms when large entries of b meet small ones of W'
+// (exact model, K = 300: entries of b and W' graded against each other over
+// one decade 2.8, two 17, three 55, four 1100 x 2^-53 of v; FP64 sums 1 to 12).
+// With 2^e, r 2^e the bound and the norm of row b, and W, R the largest bound and
+// norm of the rows of W', the root-mean-square error of v is at most
+//   2 2^-56 r 2^e (0.58 (3 2^e R + r 2^e W) + 0.82 sqrt(K) 2^e W):
+// the entries' rounding (2^-55 / sqrt(12) of their bound) in b (twice as a factor,
+// once in the sum over n, that of the epilogue below it) and in W', and the six digit
+// products of t = 7 (each sqrt(1 / 12) 2^8 twice).  Up to 2 x 2^-53 of v it
+// stands (0.7 to 1 for a dielectric matrix and normal b of any K; graded alike,
+// over four decades, 1 to 4, where the error was below 3); beyond, and where
+// anything is not finite, the DMMA kernel forms the block again.
+constexpr int REDO_ROWS = kPairRedoRows;
+struct DigitCheck {
+  const double* scale;             // [npair] 2^(e - 7)
+  const double* norm;              // [npair] r
+  const unsigned long long* most;  // [nw] {W, R}
+  double k082;                     // 0.82 sqrt(K)
+  int* count;
+  int* list;                       // w nblk + block
+};
+__global__ void __launch_bounds__(256) k_digit_rowdot_sum(const double* __restrict__ part, int np, int npair, int nw,
+                                                          double* __restrict__ v, int ldv, DigitCheck ck) {
+  __shared__ int bad[8];
+  const int w = blockIdx.y, nblk = (npair + REDO_ROWS - 1) / REDO_ROWS;
+  const double W = __longlong_as_double((long long)ck.most[2 * w]), R = __longlong_as_double((long long)ck.most[2 * w + 1]);
+  for (int p0 = blockIdx.x * blockDim.x; p0 < npair; p0 += gridDim.x * blockDim.x) {
+    const int p = p0 + threadIdx.x;
+    bool fail = false;
+    if (p < npair) {
+      double s = 0.0;
+      for (int q = 0; q < np; ++q) s += part[((size_t)q * nw + w) * npair + p];
+      const double y = 2.0 * s;
+      v[(size_t)w * ldv + p] = y;
+      const double bound = ck.scale[p] * 128.0, n2 = ck.norm[p] * bound;
+      fail = !(n2 * (0.58 * (3.0 * bound * R + n2 * W) + ck.k082 * bound * W) <= 8.0 * fabs(y));
+    }
+    const int any = __any_sync(0xffffffffu, fail);
+    if ((threadIdx.x & 31) == 0) bad[threadIdx.x >> 5] = any;
+    __syncthreads();
+    if (threadIdx.x < 256 / REDO_ROWS && (bad[2 * threadIdx.x] | bad[2 * threadIdx.x + 1]))
+      ck.list[atomicAdd(ck.count, 1)] = w * nblk + p0 / REDO_ROWS + threadIdx.x;
+    __syncthreads();
   }
 }
 
@@ -777,15 +818,40 @@ __device__ __forceinline__ unsigned long long warp_max(unsigned long long m) {
   return m;
 }
 
+// What the split finds out about the rows besides their scales (either may be
+// null): norm[r] = |row r| relative to 2^e (0 for a row that is zero or not
+// finite), and per batch the largest 2^e and the largest |row| (as bit
+// patterns, zero on entry; a NaN is larger than all).
+struct SplitStats {
+  double* norm;
+  unsigned long long* most;  // [batch][2]
+};
+
+// Sum over the TPR threads of a row (every thread of the block calls it).
+template <int TPR>
+__device__ __forceinline__ double row_sum(double v, double* red) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (TPR == 256) {
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0.0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v += red[i];
+  }
+  return v;
+}
+
 // Rows of src [batch][rows][ld] (K valid columns) -> digits
 // [batch][7][rows][ldk].  TPR threads per row, blocks of 256.  lower: only the
 // columns c <= r of row r are taken.
 template <int TPR>
 __global__ void __launch_bounds__(256) k_digit_split(const double* __restrict__ src, int rows, int K, int ld,
                                                      size_t src_stride, int lower, int8_t* __restrict__ dig, int ldk,
-                                                     double* __restrict__ scale, int lds) {
+                                                     double* __restrict__ scale, int lds, SplitStats st) {
+  static_assert(TPR == 32 || TPR == 256, "a warp or a block per row");
   constexpr int RPB = 256 / TPR;
   __shared__ unsigned long long red[8];
+  __shared__ double redd[8];
   const int r = blockIdx.x * RPB + threadIdx.x / TPR, t = threadIdx.x % TPR, w = blockIdx.y;
   const bool live = r < rows;
   const double* p = src + (size_t)w * src_stride + (size_t)(live ? r : 0) * ld;
@@ -803,18 +869,32 @@ __global__ void __launch_bounds__(256) k_digit_split(const double* __restrict__ 
 #pragma unroll
     for (int i = 0; i < 8; ++i) m = max(m, red[i]);
   }
-  if (!live) return;
   const RowScale sc = digit_scale(m);
   const size_t slab = (size_t)rows * ldk;
   int8_t* d = dig + (size_t)w * 7 * slab + (size_t)r * ldk;
   // lower: the K blocks that the row's column tile reads.
-  const int end = lower ? min(ldk, (r / dgt::TN + 1) * dgt::TN) : ldk;
+  const int end = !live ? 0 : lower ? min(ldk, (r / dgt::TN + 1) * dgt::TN) : ldk;
+  double s2 = 0.0;
   for (int k = 8 * t; k < end; k += 8 * TPR) {
     load8(p, k, lim, x);
     digit_store8(x, sc, d + k, slab);
+    if (st.norm || st.most) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const double y = sc.f1 == 0.0 ? 0.0 : x[i] * sc.f1 * sc.f2;
+        s2 = fma(y, y, s2);
+      }
+    }
   }
-  if (t == 0) {
+  if (st.norm || st.most) s2 = sqrt(row_sum<TPR>(s2, redd)) * 0x1p-55;
+  if (live && t == 0) {
     scale[(size_t)w * lds + r] = sc.sc;
+    if (st.norm) st.norm[r] = s2;
+    if (st.most) {
+      const double bound = sc.sc * 128.0;
+      atomicMax(st.most + 2 * w, (unsigned long long)__double_as_longlong(bound));
+      atomicMax(st.most + 2 * w + 1, (unsigned long long)__double_as_longlong(bound * s2));
+    }
   }
 }
 
@@ -983,12 +1063,13 @@ static bool try_reserve(DevBuf& b, size_t bytes) {
 }
 
 static void split_rows(qx_ctx* ctx, const double* src, int rows, int K, int ld, size_t stride, int batch, int lower,
-                       int8_t* dig, int ldk, double* scale, int lds) {
+                       int8_t* dig, int ldk, double* scale, int lds, SplitStats st = {nullptr, nullptr}) {
   if (K <= 2048)
     k_digit_split<32><<<dim3(ceil_div(rows, 8), batch), 256, 0, ctx->stream>>>(src, rows, K, ld, stride, lower, dig,
-                                                                             ldk, scale, lds);
+                                                                             ldk, scale, lds, st);
   else
-    k_digit_split<256><<<dim3(rows, batch), 256, 0, ctx->stream>>>(src, rows, K, ld, stride, lower, dig, ldk, scale, lds);
+    k_digit_split<256><<<dim3(rows, batch), 256, 0, ctx->stream>>>(src, rows, K, ld, stride, lower, dig, ldk, scale,
+                                                                   lds, st);
   check_launch(ctx);
 }
 
@@ -1085,26 +1166,36 @@ bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int np
   const int fc = (int)std::max<size_t>(1, std::min<size_t>(nw, budget / (row * naux)));
   int pc = (int)std::max<size_t>(256, std::min<size_t>(npair, budget / row));
   pc = std::min(round_up(pc, 256), npair);
-  const int lds = NT * dgt::TN;
+  const int lds = NT * dgt::TN, redo_cap = ceil_div(pc, REDO_ROWS) * fc;
   DevBuf &da = ctx->ws[WS_DIG_A], &db = ctx->ws[WS_DIG_B], &ds = ctx->ws[WS_DIG_S], &dp = ctx->ws[WS_DIG_P];
   if (!try_reserve(da, row * pc) || !try_reserve(db, row * naux * fc) ||
-      !try_reserve(ds, ((size_t)pc + (size_t)lds * fc) * sizeof(double)) ||
+      !try_reserve(ds, ((size_t)2 * pc + (size_t)(lds + 2) * fc + 1) * sizeof(double) + redo_cap * sizeof(int)) ||
       !try_reserve(dp, ((size_t)2 * NT * fc * pc + (size_t)round_up(pc, 256) * lds) * sizeof(double)))
     return false;
   int2* xt = reinterpret_cast<int2*>(dp.as<double>() + (size_t)2 * NT * fc * pc);
+  // Scales of W', its largest bounds and norms, the count of the blocks to form
+  // again (zeroed together), scales and norms of the pairs, the list of those blocks.
   double* sb = ds.as<double>();
-  double* sa = sb + (size_t)lds * fc;
-  QX_CUDA(cudaMemsetAsync(sb, 0, (size_t)lds * fc * sizeof(double), ctx->stream));
+  unsigned long long* most = reinterpret_cast<unsigned long long*>(sb + (size_t)lds * fc);
+  int* redo_count = reinterpret_cast<int*>(most + 2 * fc);
+  double* sa = reinterpret_cast<double*>(redo_count + 2);
+  double* norm = sa + pc;
+  int* redo = reinterpret_cast<int*>(norm + pc);
   for (int p0 = 0; p0 < npair; p0 += pc) {
     const int np = std::min(pc, npair - p0);
-    split_rows(ctx, bpt + (size_t)p0 * ldk, np, naux, ldk, 0, 1, 0, da.as<int8_t>(), ldd, sa, 0);
+    split_rows(ctx, bpt + (size_t)p0 * ldk, np, naux, ldk, 0, 1, 0, da.as<int8_t>(), ldd, sa, 0, {norm, nullptr});
     k_digit_xt<<<dim3(lds / 32, ceil_div(np, 32)), 256, 0, ctx->stream>>>(bpt + (size_t)p0 * ldk, np, naux, ldk, sa, lds,
                                                                            xt);
     check_launch(ctx);
     for (int w0 = 0; w0 < nw; w0 += fc) {
       const int n = std::min(fc, nw - w0);
-      if (p0 == 0 || fc < nw)
-        split_rows(ctx, wc + (size_t)w0 * wc_stride, naux, naux, ldn, wc_stride, n, 1, db.as<int8_t>(), ldd, sb, lds);
+      if (p0 == 0 || fc < nw) {
+        QX_CUDA(cudaMemsetAsync(sb, 0, ((size_t)(lds + 2) * fc + 1) * sizeof(double), ctx->stream));
+        split_rows(ctx, wc + (size_t)w0 * wc_stride, naux, naux, ldn, wc_stride, n, 1, db.as<int8_t>(), ldd, sb, lds,
+                   {nullptr, most});
+      } else {
+        QX_CUDA(cudaMemsetAsync(redo_count, 0, sizeof(int), ctx->stream));
+      }
       DigitArgs a{};
       a.M = np;
       a.N = naux;
@@ -1118,9 +1209,12 @@ bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int np
       a.wgroup = (int)std::max<size_t>(1, std::min<size_t>(n, ((size_t)60 << 20) / (row * naux)));
       a.part = dp.as<double>();
       launch_digit_gemm<DIGIT_ROWDOT>(ctx, da.as<int8_t>(), ldd, db.as<int8_t>(), ldd, a);
+      const DigitCheck ck{sa, norm, most, 0.82 * std::sqrt((double)naux), redo_count, redo};
       k_digit_rowdot_sum<<<dim3(std::min(ceil_div(np, 256), 512), n), 256, 0, ctx->stream>>>(
-          dp.as<double>(), 2 * NT, np, n, v + (size_t)w0 * ldv + p0, ldv);
+          dp.as<double>(), 2 * NT, np, n, v + (size_t)w0 * ldv + p0, ldv, ck);
       check_launch(ctx);
+      launch_pair_contract_redo(ctx, bpt + (size_t)p0 * ldk, ldk, np, naux, wc + (size_t)w0 * wc_stride, ldn, wc_stride,
+                                n, v + (size_t)w0 * ldv + p0, ldv, redo_count, redo);
     }
   }
   return true;

@@ -1258,18 +1258,15 @@ void launch_exchange_diag(qx_ctx* ctx, const double* lpq, int naux, int nmo, int
 // room for digits) leave SMs idle with 128 (23.5 and 44.5 us at nmo 24 and 40,
 // now 14.3 and 26.8).
 using PairTile = F64Tile<64, 64, 4, 2, 3>;
+static_assert(PairTile::BM == kPairRedoRows, "blocks of the digit kernel's list");
 
-__global__ void __launch_bounds__(PairTile::THREADS) k_pair_contract_f64(const double* __restrict__ bpt, int ldk,
-                                                                         int npair, int naux,
-                                                                         const double* __restrict__ wc, int ldn,
-                                                                         size_t wc_stride,
-                                                                         double* __restrict__ v, int ldv) {
+__device__ __forceinline__ void pair_contract_block(const double* __restrict__ bpt, int ldk, int npair, int naux,
+                                                    const double* __restrict__ wc, int ldn, size_t wc_stride,
+                                                    double* __restrict__ v, int ldv, int w, int m0) {
   using T = PairTile;
   extern __shared__ double smem[];
   __shared__ double part[T::WARPS_N][T::BM];
   __shared__ double rowacc[T::BM];
-  const int w = blockIdx.y;
-  const int m0 = blockIdx.x * T::BM;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wn = warp % T::WARPS_N;
   for (int i = threadIdx.x; i < T::BM; i += T::THREADS) rowacc[i] = 0.0;
@@ -1319,6 +1316,48 @@ __global__ void __launch_bounds__(PairTile::THREADS) k_pair_contract_f64(const d
     if (m0 + r < npair) v[(size_t)w * ldv + m0 + r] = 2.0 * rowacc[r];
 }
 
+__global__ void __launch_bounds__(PairTile::THREADS) k_pair_contract_f64(const double* __restrict__ bpt, int ldk,
+                                                                         int npair, int naux,
+                                                                         const double* __restrict__ wc, int ldn,
+                                                                         size_t wc_stride,
+                                                                         double* __restrict__ v, int ldv) {
+  pair_contract_block(bpt, ldk, npair, naux, wc, ldn, wc_stride, v, ldv, blockIdx.y, blockIdx.x * PairTile::BM);
+}
+
+// The blocks list[0 .. *count), w ceil(npair / BM) + block, one after the other.
+__global__ void __launch_bounds__(PairTile::THREADS) k_pair_contract_redo(const double* __restrict__ bpt, int ldk,
+                                                                          int npair, int naux,
+                                                                          const double* __restrict__ wc, int ldn,
+                                                                          size_t wc_stride, double* __restrict__ v,
+                                                                          int ldv, const int* __restrict__ count,
+                                                                          const int* __restrict__ list) {
+  const int n = *count, nblk = (npair + PairTile::BM - 1) / PairTile::BM;
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    const int it = list[i], w = it / nblk;
+    pair_contract_block(bpt, ldk, npair, naux, wc, ldn, wc_stride, v, ldv, w, (it - w * nblk) * PairTile::BM);
+  }
+}
+
+static void pair_attributes_once(int device) {
+  static PerDeviceOnce attr_once;
+  attr_once(device, [&] {
+    const int smem = (int)PairTile::SMEM;
+    QX_CUDA(cudaFuncSetAttribute(k_pair_contract_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    QX_CUDA(cudaFuncSetAttribute(k_pair_contract_redo, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  });
+}
+
+// Two blocks per SM go through the list; an empty one costs the launch.
+void launch_pair_contract_redo(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc, int ldn,
+                               size_t wc_stride, int nw, double* v, int ldv, const int* count, const int* list) {
+  using T = PairTile;
+  pair_attributes_once(ctx->device);
+  const long long items = (long long)ceil_div(npair, T::BM) * nw;
+  k_pair_contract_redo<<<(unsigned)std::min<long long>(items, 2 * ctx->sm_count), T::THREADS, T::SMEM, ctx->stream>>>(
+      bpt, ldk, npair, naux, wc, ldn, wc_stride, v, ldv, count, list);
+  check_launch(ctx);
+}
+
 void launch_pair_contract_fp64(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc,
                                int ldn, size_t wc_stride, int nw, double* v, int ldv) {
   // The integer tensor pipe above one column tile: with 24 frequencies the
@@ -1329,10 +1368,7 @@ void launch_pair_contract_fp64(qx_ctx* ctx, const double* bpt, int ldk, int npai
   if (naux > 160 && launch_pair_contract_digits(ctx, bpt, ldk, npair, naux, wc, ldn, wc_stride, nw, v, ldv))
     return;
   using T = PairTile;
-  static PerDeviceOnce attr_once;
-  attr_once(ctx->device, [&] {
-    QX_CUDA(cudaFuncSetAttribute(k_pair_contract_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM));
-  });
+  pair_attributes_once(ctx->device);
   dim3 grid(ceil_div(npair, T::BM), nw);
   k_pair_contract_f64<<<grid, T::THREADS, T::SMEM, ctx->stream>>>(bpt, ldk, npair, naux, wc, ldn, wc_stride, v, ldv);
   check_launch(ctx);

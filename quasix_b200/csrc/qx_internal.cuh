@@ -262,6 +262,11 @@ bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int n
                        double* eps, int ldn, size_t eps_stride);
 bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc,
                                  int ldn, size_t wc_stride, int nw, double* v, int ldv);
+// The DMMA contraction of the listed blocks of kPairRedoRows pairs (device list and
+// count), which the digits may not hold.
+constexpr int kPairRedoRows = 64;
+void launch_pair_contract_redo(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc, int ldn,
+                               size_t wc_stride, int nw, double* v, int ldv, const int* count, const int* list);
 bool gemm_nt_digits(qx_ctx* ctx, const double* A, int M, int lda, const double* B, int N, int ldb, int K, double* C,
                     int ldc);
 

@@ -1,0 +1,101 @@
+"""Operands that fixed point does not suit: the digit kernels' results stand only
+where their error is that of FP64 sums, the rest is formed by the DMMA kernels.
+
+These tests call the library's internal launchers, since through the entry
+points the inversion's own rounding hides what a contraction loses on a screened
+interaction of small entries.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CONTRACT = "_ZN2qx25launch_pair_contract_fp64EP6qx_ctxPKdiiiS3_imiPdi"
+
+
+@pytest.fixture(scope="module")
+def env():
+    import torch
+    from quasix_b200 import _native
+    ctx = _native.Context()
+    yield torch, ctx
+    ctx.close()
+
+
+def _ptr(t):
+    return C.c_void_p(t.data_ptr())
+
+
+def _pad(a, ld):
+    out = np.zeros(a.shape[:-1] + (ld,))
+    out[..., :a.shape[-1]] = a
+    return out
+
+
+def contract(env, b, wl):
+    """v[w][p] = 2 sum_n b[p][n] sum_k<=n wl[w][n][k] b[p][k]"""
+    torch, ctx = env
+    (P, K), nw = b.shape, wl.shape[0]
+    ld = (K + 7) // 8 * 8
+    tb, tw = (torch.from_numpy(_pad(x, ld)).cuda() for x in (b, wl))
+    v = torch.full((nw, P), 7.0, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    getattr(ctx.lib, CONTRACT)(ctx.handle, _ptr(tb), C.c_int(ld), C.c_int(P), C.c_int(K), _ptr(tw), C.c_int(ld),
+                               C.c_size_t(K * ld), C.c_int(nw), _ptr(v), C.c_int(P))
+    torch.cuda.synchronize()
+    return v.cpu().numpy()
+
+
+def contract_exact(b, wl):
+    """In extended precision (64-bit mantissa)."""
+    bl, w = b.astype(np.longdouble), wl.astype(np.longdouble)
+    return np.stack([2 * (bl * (bl @ np.tril(x).T)).sum(1) for x in w])
+
+
+def definite(rng, K, g, nw):
+    """Half-lower forms of -M M^T scaled by g on both sides."""
+    out = []
+    for _ in range(nw):
+        m = rng.normal(size=(K, K))
+        w = -(m @ m.T) / K * np.outer(g, g)
+        out.append(np.tril(w, -1) + np.diag(np.diag(w)) / 2)
+    return np.stack(out)
+
+
+@pytest.mark.parametrize("K,P,decades", [(161, 5, 0), (300, 64, 4), (300, 65, 6), (420, 130, 8), (180, 300, -4)])
+def test_contraction_of_opposite_grading(env, K, P, decades):
+    """Entries of b up where those of W' are down (and alike, negative), one pair
+    in three flat.  v = -|M^T g b|^2 has no cancellation beyond its sums': random
+    partial sums of K terms round at up to 2^-53 |v| each, K / 4 of them in C and
+    K / 4 in v, with 6 standard deviations 6 sqrt(K / 2) 2^-53 |v|; digits that
+    stand add their own two (12 with the same allowance)."""
+    rng = np.random.default_rng(K + P)
+    g = 10.0 ** (-abs(decades) * rng.uniform(size=K))
+    wl = definite(rng, K, g, 3)
+    b = rng.normal(size=(P, K))
+    graded = np.arange(P) % 3 > 0
+    b[graded] *= g if decades < 0 else 1 / g
+    got, ref = contract(env, b, wl), contract_exact(b, wl)
+    err = np.abs((got - ref) / ref).astype(float) * 2.0 ** 53
+    assert err.max() < 6 * np.sqrt(K / 2) + 12
+    # Not finite in one pair: that pair only.
+    b[3, 7] = np.inf
+    again = contract(env, b, wl)
+    assert not np.isfinite(again[:, 3]).any()
+    keep = np.arange(P) != 3
+    assert (np.abs((again - ref) / ref).astype(float)[:, keep] * 2.0 ** 53).max() < 6 * np.sqrt(K / 2) + 12
+
+
+def test_contraction_of_zeros(env):
+    rng = np.random.default_rng(1)
+    wl = definite(rng, 200, np.ones(200), 2)
+    b = rng.normal(size=(70, 200))
+    b[5] = 0.0
+    wl[1] = 0.0
+    wl[0, 9] = 0.0
+    got, ref = contract(env, b, wl), contract_exact(b, wl)
+    assert (got[:, 5] == 0).all() and (got[1] == 0).all()
+    err = np.abs(got[0] - ref[0])[np.arange(70) != 5] / np.abs(ref[0])[np.arange(70) != 5]
+    assert err.astype(float).max() * 2.0 ** 53 < 6 * np.sqrt(100) + 12
