@@ -93,6 +93,9 @@ struct DigitArgs {
   // onto what out holds, for a further range of K, no delta), or all tiles (wide:
   // out and ldo allow 32-byte stores).
   int lower, add, wide;
+  // lower: A is the batched operand too (scaleA = scaleB).
+  const int* skip;      // nothing to do once *skip reaches skip_at (null: never)
+  int skip_at;
   double* out;
   int ldo;
   size_t out_stride;
@@ -359,6 +362,7 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
     if (threadIdx.x == 0) atomicCAS(args.err, 0, 40);
     return;
   }
+  if (MODE != DIGIT_ROWDOT && args.skip && *args.skip >= args.skip_at) return;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + P::BAR_OFF);
@@ -419,7 +423,7 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
         if (leader) mbar_expect_tx(&full[s], 2 * P::SLOT_BYTES);
         const uint32_t dst = smem_u32(smem + s * P::SLOT_BYTES);
         const uint32_t fb = full_leader + s * 8;
-        tma_load_3d_pair(dst, &mapA, fb, kb * P::BK, t.mb * P::TM, slice);
+        tma_load_3d_pair(dst, &mapA, fb, kb * P::BK, t.mb * P::TM, (MODE == DIGIT_LOWER ? t.w * P::NS : 0) + slice);
         tma_load_3d_pair(dst + P::A_BYTES, &mapB, fb, kb * P::BK, t.nt * P::TN + (P::TN / 2) * rank,
                          t.w * P::NS + slice);
         if (++s == P::SLOTS) {
@@ -554,7 +558,7 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
       }
       drain([&](int c, int d) { s[c] = ((s[c] + half_unit) >> args.sh) + ((long long)d << (40 - args.sh)); });
       if (!ok) break;
-      const double sa = m < args.M ? args.scaleA[m] : 0.0;
+      const double sa = m < args.M ? args.scaleA[MODE == DIGIT_LOWER ? (size_t)t.w * args.ldsb + m : m] : 0.0;
       if (MODE == DIGIT_ROWDOT) {
         // Each thread contracts its row of C with its row of X, in integers:
         // FP64 instructions get next to no issue slots while the MMAs run at
@@ -739,29 +743,50 @@ __global__ void __launch_bounds__(256) k_digit_rowdot_sum(const double* __restri
 struct RowScale {
   double f1, f2, sc;
 };
-__device__ __forceinline__ RowScale digit_scale(unsigned long long amax) {
+constexpr int kNotFinite = 1 << 30;
+// f1 and f2 from k = 55 - e (kNotFinite: zeros).
+__device__ __forceinline__ RowScale scale_factors(int k) {
   RowScale r;
+  const int k1 = k >> 1;
+  r.f1 = k == kNotFinite ? 0.0 : pow2i(k1);
+  r.f2 = k == kNotFinite ? 0.0 : pow2i(k - k1);
+  r.sc = 0.0;
+  return r;
+}
+__device__ __forceinline__ int digit_scale(unsigned long long amax, double& sc) {
   if (amax >= 0x7FF0000000000000ull) {
-    r.f1 = r.f2 = 0.0;
-    r.sc = __longlong_as_double(0x7FF8000000000000ll);
-    return r;
+    sc = __longlong_as_double(0x7FF8000000000000ll);
+    return kNotFinite;
   }
   if (amax == 0) {
-    r.f1 = r.f2 = 1.0;
-    r.sc = 0.0;
-    return r;
+    sc = 0.0;
+    return 55;
   }
   int e = max(1, (int)(amax >> 52)) - 1022;
   if ((amax & 0xFFFFFFFFFFFFFull) >= 0xFC00000000000ull) ++e;
-  const int k = 55 - e, k1 = k >> 1;
-  r.f1 = pow2i(k1);
-  r.f2 = pow2i(k - k1);
-  r.sc = ldexp(1.0, e - 7);
+  sc = ldexp(1.0, e - 7);
+  return 55 - e;
+}
+__device__ __forceinline__ RowScale digit_scale(unsigned long long amax) {
+  double sc;
+  RowScale r = scale_factors(digit_scale(amax, sc));
+  r.sc = sc;
   return r;
 }
 
 // Eight entries (as their 56-bit integers) -> eight bytes of each digit slice.
-__device__ __forceinline__ void digit_store8(const double (&x)[8], const RowScale& r, int8_t* dst, size_t slab) {
+// What is seen of a row while it is split: the sum of squares of its top digits
+// (x ~ d_0 2^(e - 7)), and the entries without one (below 2^(e - 8)).
+struct TopDigits {
+  int squares = 0, zeros = 0;
+  __device__ __forceinline__ void add(uint32_t four) {
+    squares = __dp4a((int)four, (int)four, squares);
+    zeros += __popc(~(((four & 0x7f7f7f7fu) + 0x7f7f7f7fu) | four) & 0x80808080u);
+  }
+};
+
+__device__ __forceinline__ void digit_store8(const double (&x)[8], const RowScale& r, int8_t* dst, size_t slab,
+                                             TopDigits& top) {
   constexpr unsigned long long BIAS = 0x80808080808080ull;
   uint32_t lo[8], hi[8];
 #pragma unroll
@@ -787,6 +812,7 @@ __device__ __forceinline__ void digit_store8(const double (&x)[8], const RowScal
     w[5][h] = __byte_perm(t0, t1, 0x7632);
     t0 = __byte_perm(g[0], g[1], 0x7362), t1 = __byte_perm(g[2], g[3], 0x7362);
     w[6][h] = __byte_perm(t0, t1, 0x5410);
+    top.add(w[6][h]);
   }
 #pragma unroll
   for (int i = 0; i < 7; ++i)
@@ -820,8 +846,8 @@ __device__ __forceinline__ unsigned long long warp_max(unsigned long long m) {
 }
 
 // What the split finds out about the rows besides their scales (either may be
-// null): norm[r] = |row r| relative to 2^e (0 for a row that is zero or not
-// finite), and per batch the largest 2^e and the largest |row| (as bit
+// null): norm[r], |row r| relative to 2^e, from above (the top digits' and their
+// rounding's); and per batch the largest 2^e and the largest |row| (as bit
 // patterns, zero on entry; a NaN is larger than all).
 struct SplitStats {
   double* norm;
@@ -830,16 +856,15 @@ struct SplitStats {
 
 // Sum over the TPR threads of a row (every thread of the block calls it).
 template <int TPR>
-__device__ __forceinline__ double row_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (TPR == 256) {
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    v = 0.0;
+__device__ __forceinline__ long long row_sum(int v, int* red) {
+  v = __reduce_add_sync(0xffffffffu, v);
+  if (TPR == 32) return v;
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  long long s = 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v += red[i];
-  }
-  return v;
+  for (int i = 0; i < 8; ++i) s += red[i];
+  return s;
 }
 
 // Rows of src [batch][rows][ld] (K valid columns) -> digits
@@ -852,7 +877,7 @@ __global__ void __launch_bounds__(256) k_digit_split(const double* __restrict__ 
   static_assert(TPR == 32 || TPR == 256, "a warp or a block per row");
   constexpr int RPB = 256 / TPR;
   __shared__ unsigned long long red[8];
-  __shared__ double redd[8];
+  __shared__ int redi[8];
   const int r = blockIdx.x * RPB + threadIdx.x / TPR, t = threadIdx.x % TPR, w = blockIdx.y;
   const bool live = r < rows;
   const double* p = src + (size_t)w * src_stride + (size_t)(live ? r : 0) * ld;
@@ -875,26 +900,19 @@ __global__ void __launch_bounds__(256) k_digit_split(const double* __restrict__ 
   int8_t* d = dig + (size_t)w * 7 * slab + (size_t)r * ldk;
   // lower: the K blocks that the row's column tile reads.
   const int end = !live ? 0 : lower ? min(ldk, (r / dgt::TN + 1) * dgt::TN) : ldk;
-  double s2 = 0.0;
+  TopDigits top;
   for (int k = 8 * t; k < end; k += 8 * TPR) {
     load8(p, k, lim, x);
-    digit_store8(x, sc, d + k, slab);
-    if (st.norm || st.most) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const double y = sc.f1 == 0.0 ? 0.0 : x[i] * sc.f1 * sc.f2;
-        s2 = fma(y, y, s2);
-      }
-    }
+    digit_store8(x, sc, d + k, slab, top);
   }
-  if (st.norm || st.most) s2 = sqrt(row_sum<TPR>(s2, redd)) * 0x1p-55;
+  const double squares = (double)row_sum<TPR>(top.squares, redi);
   if (live && t == 0) {
     scale[(size_t)w * lds + r] = sc.sc;
-    if (st.norm) st.norm[r] = s2;
+    const double norm = (sqrt(squares) + 0.5 * sqrt((double)lim)) * 0x1p-7, bound = sc.sc * 128.0;
+    if (st.norm) st.norm[r] = norm;
     if (st.most) {
-      const double bound = sc.sc * 128.0;
       atomicMax(st.most + 2 * w, (unsigned long long)__double_as_longlong(bound));
-      atomicMax(st.most + 2 * w + 1, (unsigned long long)__double_as_longlong(bound * s2));
+      atomicMax(st.most + 2 * w + 1, (unsigned long long)__double_as_longlong(bound * norm));
     }
   }
 }
@@ -924,45 +942,85 @@ __global__ void __launch_bounds__(256) k_digit_xt(const double* __restrict__ b, 
   }
 }
 
-// Digits of b[P][k] chi[w][k] for DG_R rows and DG_F frequencies per block:
-// the row is read from L2 once for the frequencies, chi once for the rows.
+// Rows that fixed point does not suit, by blocks of 64: block[w nblk + r / 64]
+// (zero on entry) and the number of blocks marked.
+//
+// The rounding of an entry (2^-55 of the bound 2^e) and the dropped digit products
+// make an error of a product of two rows, in 2^-53 of the root-sum-square of its
+// terms, of about rho rho' / 10, rho = 2^e / rms.  The DMMA kernel's sums of K
+// random terms make 0.28 sqrt(K).  A row stands for its digits up to rho = 2.5
+// K^(1/4), and while at most twice as many of its entries have a zero top digit,
+// |x| < 2^(e - 8), as of a normal row (0.8 rho / 256 of them; weighted ones 1.3, and the
+// margin of a small K): two such rows share most of their large entries.
+// Measured for normal B and the weights of zero frequency, digits / DMMA, rms over the
+// elements: K = 1024 4.6 / 8.5, 2020 5.5 / 12, 5270 5.9 / 19, 10 400 7.1 / 28.  In an
+// exact model, K = 10 400: an entry of 30 rms in a row (marked) 42; rows of
+// log-uniform entries over one decade, up where the other's are down, 24, over one
+// and a half (marked, as all that follow) 73, over four 2 10^4.
+constexpr int ROUGH_ROWS = kRoughRows;
+struct RoughRows {
+  int* block;
+  int* count;
+  int nblk;
+};
+// A row's scale 2^(e - 7), sum of squares and number of zeros of its K top digits.
+__device__ __forceinline__ void mark_rough(const RoughRows& g, int w, int r, double scale, long long squares, int zeros,
+                                           int K) {
+  if (scale == 0.0) return;
+  const double k2 = sqrt((double)K), rho = 128.0 * k2 / sqrt((double)squares);
+  if (isfinite(scale) && rho <= 2.5 * sqrt(k2) && zeros <= 0x1p-8 * 1.6 * rho * K + 0.5 * k2) return;
+  if (atomicExch(g.block + (size_t)w * g.nblk + r / ROUGH_ROWS, 1) == 0) atomicAdd(g.count, 1);
+}
+
+// Digits of b[P][k] sqrt(chi[w][k]) for DG_R rows and DG_F frequencies per block:
+// the row is read from L2 once for the frequencies, root = sqrt(chi) once for the
+// rows.  The weights go to both operands of P0 by halves, which are then one: all on
+// one side its rows have larger bounds (normal rows, zero frequency, K = 5270:
+// 8.6 x 2^-53 instead of 6.3, for the DMMA's 9.9), and B_ov is split as well.
 constexpr int DG_R = 2, DG_F = 4;
-__global__ void __launch_bounds__(256) k_digit_split_chi(const double* __restrict__ b, int rows, int K, int ld,
-                                                         const double* __restrict__ chi, int ldchi, int nw,
+__global__ void __launch_bounds__(256, 2) k_digit_split_chi(const double* __restrict__ b, int rows, int K, int ld,
+                                                         const double* __restrict__ root, int ldr, int nw,
                                                          int8_t* __restrict__ dig, int ldk,
-                                                         double* __restrict__ scale, int lds) {
-  __shared__ unsigned long long red[8][DG_R * DG_F];
+                                                         double* __restrict__ scale, int lds, RoughRows rough) {
+  constexpr int NC = DG_R * DG_F;
+  __shared__ unsigned long long red[8][NC], squares[NC];
+  __shared__ int zeros[NC];
   const int r0 = blockIdx.x * DG_R, w0 = blockIdx.y * DG_F;
   const int nr = min(DG_R, rows - r0), nf = min(DG_F, nw - w0);
-  unsigned long long m[DG_R * DG_F];
+  unsigned long long m[NC];
 #pragma unroll
-  for (int i = 0; i < DG_R * DG_F; ++i) m[i] = 0;
+  for (int i = 0; i < NC; ++i) m[i] = 0;
   for (int k = 8 * threadIdx.x; k < K; k += 8 * 256) {
     double x[DG_R][8], c[8];
 #pragma unroll
     for (int r = 0; r < DG_R; ++r) load8(b + (size_t)(r0 + min(r, nr - 1)) * ld, k, K, x[r]);
 #pragma unroll
     for (int f = 0; f < DG_F; ++f) {
-      load8(chi + (size_t)(w0 + min(f, nf - 1)) * ldchi, k, K, c);
+      load8(root + (size_t)(w0 + min(f, nf - 1)) * ldr, k, K, c);
 #pragma unroll
       for (int r = 0; r < DG_R; ++r)
 #pragma unroll
         for (int i = 0; i < 8; ++i) m[r * DG_F + f] = max(m[r * DG_F + f], abs_bits(x[r][i] * c[i]));
     }
   }
+  if (threadIdx.x < NC) squares[threadIdx.x] = zeros[threadIdx.x] = 0;
 #pragma unroll
-  for (int i = 0; i < DG_R * DG_F; ++i) {
+  for (int i = 0; i < NC; ++i) {
     const unsigned long long v = warp_max(m[i]);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][i] = v;
   }
   __syncthreads();
-  RowScale sc[DG_R * DG_F];
+  int kexp[NC];
+  TopDigits top[NC];
+  double my_scale = 0.0;  // of combination threadIdx.x
 #pragma unroll
-  for (int i = 0; i < DG_R * DG_F; ++i) {
+  for (int i = 0; i < NC; ++i) {
     unsigned long long v = 0;
+    double scale_i;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) v = max(v, red[q][i]);
-    sc[i] = digit_scale(v);
+    for (int j = 0; j < 8; ++j) v = max(v, red[j][i]);
+    kexp[i] = digit_scale(v, scale_i);
+    if (threadIdx.x == i) my_scale = scale_i;
   }
   const size_t slab = (size_t)rows * ldk;
   for (int k = 8 * threadIdx.x; k < ldk; k += 8 * 256) {
@@ -972,22 +1030,40 @@ __global__ void __launch_bounds__(256) k_digit_split_chi(const double* __restric
 #pragma unroll
     for (int f = 0; f < DG_F; ++f) {
       if (f >= nf) break;
-      load8(chi + (size_t)(w0 + f) * ldchi, k, K, c);
+      load8(root + (size_t)(w0 + f) * ldr, k, K, c);
 #pragma unroll
       for (int r = 0; r < DG_R; ++r) {
         if (r >= nr) break;
 #pragma unroll
         for (int i = 0; i < 8; ++i) y[i] = x[r][i] * c[i];
-        digit_store8(y, sc[r * DG_F + f], dig + (size_t)(w0 + f) * 7 * slab + (size_t)(r0 + r) * ldk + k, slab);
+        digit_store8(y, scale_factors(kexp[r * DG_F + f]), dig + (size_t)(w0 + f) * 7 * slab + (size_t)(r0 + r) * ldk + k,
+                     slab, top[r * DG_F + f]);
       }
     }
   }
-  if (threadIdx.x < DG_R * DG_F) {
-    const int r = threadIdx.x / DG_F, f = threadIdx.x % DG_F;
-    unsigned long long v = 0;
-    for (int q = 0; q < 8; ++q) v = max(v, red[q][threadIdx.x]);
-    if (r < nr && f < nf) scale[(size_t)(w0 + f) * lds + r0 + r] = digit_scale(v).sc;
+#pragma unroll
+  for (int i = 0; i < NC; ++i) {
+    const int q = __reduce_add_sync(0xffffffffu, top[i].squares), n = __reduce_add_sync(0xffffffffu, top[i].zeros);
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&squares[i], (unsigned long long)q);
+      atomicAdd(&zeros[i], n);
+    }
   }
+  __syncthreads();
+  if (threadIdx.x < NC) {
+    const int r = threadIdx.x / DG_F, f = threadIdx.x % DG_F;
+    if (r < nr && f < nf) {
+      scale[(size_t)(w0 + f) * lds + r0 + r] = my_scale;
+      // (less the zeros from K to ldk)
+      mark_rough(rough, w0 + f, r0 + r, my_scale, (long long)squares[threadIdx.x], zeros[threadIdx.x] - (ldk - K), K);
+    }
+  }
+}
+
+// root[w][k] = sqrt(chi[w][k])
+__global__ void k_digit_root(const double* __restrict__ chi, size_t n, double* __restrict__ root) {
+  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
+    root[k] = sqrt(chi[k]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1013,7 +1089,7 @@ template <int MODE>
 static void launch_digit_gemm(qx_ctx* ctx, const int8_t* a, int lda, const int8_t* b, int ldb, DigitArgs args) {
   args.rowdot = MODE == DIGIT_ROWDOT;
   args.lower = MODE == DIGIT_LOWER;
-  const CUtensorMap ma = digit_map(a, args.K, args.M, lda, dgt::NS, dgt::TM);
+  const CUtensorMap ma = digit_map(a, args.K, args.M, lda, MODE == DIGIT_LOWER ? dgt::NS * args.nbatch : dgt::NS, dgt::TM);
   const CUtensorMap mb = digit_map(b, args.K, args.N, ldb, dgt::NS * args.nbatch, dgt::TN / 2);
   QX_REQUIRE(args.K > 0 && args.K <= dgt::KMAX, QX_ERR_INVALID_INPUT, "digit GEMM: K = %d", args.K);
   args.sh = 0;
@@ -1078,41 +1154,52 @@ static void split_rows(qx_ctx* ctx, const double* src, int rows, int K, int ld, 
 // launch); larger problems run in chunks.  Batch workers share the device.
 static size_t digit_budget(qx_ctx* ctx) { return ctx->worker ? (size_t)512 << 20 : (size_t)1536 << 20; }
 
-// eps[w] = I + B_ov diag(chi'[w]) B_ov^T.
+// eps[w] = I + B_ov diag(chi'[w]) B_ov^T, chi' >= 0.
 bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw,
                        double* eps, int ldn, size_t eps_stride) {
   const int ldk = round_up(nov, 16);
-  const size_t a_bytes = (size_t)7 * naux * ldk;
-  const int fmax = (int)std::max<size_t>(1, std::min<size_t>(nw, digit_budget(ctx) / a_bytes));
+  const size_t per = (size_t)7 * naux * ldk;
+  const int fmax = (int)std::max<size_t>(1, std::min<size_t>(nw, digit_budget(ctx) / per));
   const int chunks = ceil_div(nw, fmax), fc = ceil_div(nw, chunks);
-  DevBuf &da = ctx->ws[WS_DIG_A], &db = ctx->ws[WS_DIG_B], &ds = ctx->ws[WS_DIG_S];
-  const int lds = round_up(naux, dgt::TN);
-  if (!try_reserve(da, a_bytes) || !try_reserve(db, a_bytes * fc) ||
-      !try_reserve(ds, ((size_t)naux + (size_t)lds * fc) * sizeof(double)))
+  DevBuf &db = ctx->ws[WS_DIG_B], &ds = ctx->ws[WS_DIG_S];
+  const int lds = round_up(naux, dgt::TN), nblk = ceil_div(naux, ROUGH_ROWS);
+  const size_t n_scale = (size_t)lds * fc, n_flag = (size_t)nblk * fc + 1, n_root = (size_t)ldov * fc;
+  if (!try_reserve(db, per * fc) ||
+      !try_reserve(ds, (n_root + n_scale) * sizeof(double) + n_flag * sizeof(int)))
     return false;
-  double* sb = ds.as<double>();
-  double* sa = sb + (size_t)lds * fc;
-  QX_CUDA(cudaMemsetAsync(sb, 0, (size_t)lds * fc * sizeof(double), ctx->stream));
-  split_rows(ctx, bov, naux, nov, ldov, 0, 1, 0, da.as<int8_t>(), ldk, sa, 0);
+  // Roots of the weights; scales, the number of marked blocks and the blocks (zeroed together).
+  double* root = ds.as<double>();
+  double* sb = root + n_root;
+  int* marked = reinterpret_cast<int*>(sb + n_scale);
+  const RoughRows rough{marked + 1, marked, nblk};
   for (int w0 = 0; w0 < nw; w0 += fc) {
     const int n = std::min(fc, nw - w0);
+    QX_CUDA(cudaMemsetAsync(sb, 0, n_scale * sizeof(double) + n_flag * sizeof(int), ctx->stream));
+    const size_t nr = (size_t)n * ldov;
+    k_digit_root<<<(unsigned)std::min<size_t>((nr + 255) / 256, 2048), 256, 0, ctx->stream>>>(
+        chi + (size_t)w0 * ldov, nr, root);
+    check_launch(ctx);
     k_digit_split_chi<<<dim3(ceil_div(naux, DG_R), ceil_div(n, DG_F)), 256, 0, ctx->stream>>>(
-        bov, naux, nov, ldov, chi + (size_t)w0 * ldov, ldov, n, db.as<int8_t>(), ldk, sb, lds);
+        bov, naux, nov, ldov, root, ldov, n, db.as<int8_t>(), ldk, sb, lds, rough);
     check_launch(ctx);
     DigitArgs a{};
     a.M = a.N = naux;
     a.nbatch = n;
-    a.scaleA = sa;
-    a.scaleB = sb;
+    a.scaleA = a.scaleB = sb;
     a.ldsb = lds;
     a.out = eps + (size_t)w0 * eps_stride;
     a.ldo = ldn;
     a.out_stride = eps_stride;
+    a.skip = marked;
+    a.skip_at = nblk * n;
     for (int k0 = 0; k0 < nov; k0 += dgt::KMAX) {
       a.K = std::min(dgt::KMAX, nov - k0);
       a.add = k0 > 0;
-      launch_digit_gemm<DIGIT_LOWER>(ctx, da.as<int8_t>() + k0, ldk, db.as<int8_t>() + k0, ldk, a);
+      launch_digit_gemm<DIGIT_LOWER>(ctx, db.as<int8_t>() + k0, ldk, db.as<int8_t>() + k0, ldk, a);
     }
+    // The tiles with marked rows by the DMMA kernel.
+    launch_eps_dmma(ctx, bov, ldov, naux, nov, chi + (size_t)w0 * ldov, n, eps + (size_t)w0 * eps_stride, ldn,
+                    eps_stride, rough.block);
   }
   return true;
 }

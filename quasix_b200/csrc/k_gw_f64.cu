@@ -46,11 +46,12 @@ void launch_chi(qx_ctx* ctx, const double* energies, int nocc, int nvir, const d
 // Eight warps of 16 x 32 (four of 32 x 32 left the FP64 tensor pipe waiting on
 // its operands: 22.5 us at naux 139 / nov 352, now 18.1; a batch 658 -> 572 us).
 using EpsTile = F64Tile<64, 64, 4, 2, 3>;
+static_assert(EpsTile::BM == kRoughRows && EpsTile::BN == kRoughRows, "blocks of marked rows");
 
 __global__ void __launch_bounds__(EpsTile::THREADS) k_eps_f64(const double* __restrict__ bov, int ldov, int naux,
                                                               int nov, const double* __restrict__ chi,
                                                               double* __restrict__ eps, int ldn,
-                                                              size_t eps_stride) {
+                                                              size_t eps_stride, const int* __restrict__ rough) {
   using T = EpsTile;
   extern __shared__ double smem[];
   // Lower-triangular tile index -> (tm, tn), tm >= tn.
@@ -61,6 +62,10 @@ __global__ void __launch_bounds__(EpsTile::THREADS) k_eps_f64(const double* __re
   const int tn = t - tm * (tm + 1) / 2;
   const int w = blockIdx.y;
   const int m0 = tm * T::BM, n0 = tn * T::BN;
+  if (rough) {
+    const int* g = rough + (size_t)w * ((naux + T::BM - 1) / T::BM);
+    if (!(g[tm] | g[tn])) return;
+  }
   double acc[T::MI][T::NJ][2];
 #pragma unroll
   for (int i = 0; i < T::MI; ++i)
@@ -76,10 +81,10 @@ __global__ void __launch_bounds__(EpsTile::THREADS) k_eps_f64(const double* __re
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int m = m0 + f64_row<T>(i), n = n0 + f64_col<T>(j, e);
-        if (m < naux && n < naux) {
+        if (m < naux && n <= m) {  // and its mirror: exactly symmetric
           const double v = acc[i][j][e] + (m == n ? 1.0 : 0.0);
           E[(size_t)m * ldn + n] = v;
-          if (tm != tn) E[(size_t)n * ldn + m] = v;
+          if (m != n) E[(size_t)n * ldn + m] = v;
         }
       }
 }
@@ -88,13 +93,18 @@ void launch_eps_fp64(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov
                      double* eps, int ldn, size_t eps_stride, int smooth) {
   // The integer tensor pipe from where it is the faster one: with 24
   // frequencies P0 took 137 (DMMA) and 152 us (digits) at naux 300 / nov 949,
-  // 295 and 209 us at 350 / 1411, 474 and 264 us at 423 / 2020.  Its digits are
-  // relative to the largest entry of a row of B_ov chi': only for weights that
-  // do not differ too much (smooth), and for K long enough for its error (which
-  // grows as sqrt(K), the DMMA's as K) to be the smaller one in any case.
+  // 295 and 209 us at 350 / 1411, 474 and 264 us at 423 / 2020.  Only for positive
+  // weights that do not differ too much (smooth); from K = 1024 on its error is
+  // half the DMMA's or less, and rows that fixed point does not suit come back
+  // here (k_digits.cu has both figures).
   if (smooth && naux >= 256 && nov >= 1024 &&
       launch_eps_digits(ctx, bov, ldov, naux, nov, chi, nw, eps, ldn, eps_stride))
     return;
+  launch_eps_dmma(ctx, bov, ldov, naux, nov, chi, nw, eps, ldn, eps_stride, nullptr);
+}
+
+void launch_eps_dmma(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw, double* eps,
+                     int ldn, size_t eps_stride, const int* rough) {
   using T = EpsTile;
   const int tiles = ceil_div(naux, T::BM);
   dim3 grid(tiles * (tiles + 1) / 2, nw);
@@ -102,7 +112,7 @@ void launch_eps_fp64(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov
   attr_once(ctx->device, [&] {
     QX_CUDA(cudaFuncSetAttribute(k_eps_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM));
   });
-  k_eps_f64<<<grid, T::THREADS, T::SMEM, ctx->stream>>>(bov, ldov, naux, nov, chi, eps, ldn, eps_stride);
+  k_eps_f64<<<grid, T::THREADS, T::SMEM, ctx->stream>>>(bov, ldov, naux, nov, chi, eps, ldn, eps_stride, rough);
   check_launch(ctx);
 }
 

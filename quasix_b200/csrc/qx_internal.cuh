@@ -262,6 +262,11 @@ bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int n
                        double* eps, int ldn, size_t eps_stride);
 bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc,
                                  int ldn, size_t wc_stride, int nw, double* v, int ldv);
+// P0 by the DMMA kernel; rough (or null): only the tiles with a marked block of
+// kRoughRows rows, rough[w ceil(naux / kRoughRows) + block].
+constexpr int kRoughRows = 64;
+void launch_eps_dmma(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw, double* eps,
+                     int ldn, size_t eps_stride, const int* rough);
 // The DMMA contraction of the listed blocks of kPairRedoRows pairs (device list and
 // count), which the digits may not hold.
 constexpr int kPairRedoRows = 64;

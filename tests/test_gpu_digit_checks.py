@@ -12,6 +12,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+P0 = "_ZN2qx15launch_eps_fp64EP6qx_ctxPKdiiiS3_iPdimi"
 CONTRACT = "_ZN2qx25launch_pair_contract_fp64EP6qx_ctxPKdiiiS3_imiPdi"
 
 
@@ -99,3 +100,57 @@ def test_contraction_of_zeros(env):
     assert (got[:, 5] == 0).all() and (got[1] == 0).all()
     err = np.abs(got[0] - ref[0])[np.arange(70) != 5] / np.abs(ref[0])[np.arange(70) != 5]
     assert err.astype(float).max() * 2.0 ** 53 < 6 * np.sqrt(100) + 24
+
+
+def p0(env, b, chi):
+    """eps[w] = I + b diag(chi[w]) b^T"""
+    torch, ctx = env
+    (N, K), nw = b.shape, chi.shape[0]
+    ldk, ldn = (K + 7) // 8 * 8, (N + 7) // 8 * 8
+    tb, tc = (torch.from_numpy(_pad(x, ldk)).cuda() for x in (b, chi))
+    eps = torch.zeros((nw, N, ldn), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    getattr(ctx.lib, P0)(ctx.handle, _ptr(tb), C.c_int(ldk), C.c_int(N), C.c_int(K), _ptr(tc), C.c_int(nw), _ptr(eps),
+                         C.c_int(ldn), C.c_size_t(N * ldn), C.c_int(1))
+    torch.cuda.synchronize()
+    return eps.cpu().numpy()[:, :, :N]
+
+
+@pytest.mark.parametrize("N,K,rows", [(256, 1023, "normal"), (256, 1024, "normal"), (300, 1100, "normal"),
+                                      (511, 1031, "normal"), (257, 1030, "opposite"), (320, 1040, "some opposite"),
+                                      (300, 1024, "outliers"), (256, 1025, "zeros")])
+def test_p0_of_rough_rows(env, N, K, rows):
+    """Rows of B graded over four decades, half of them up where the others are
+    down; large single entries; empty rows.  In 2^-53 of the root-sum-square of an
+    element's terms: FP64 sums err by 0.3 sqrt(K) (k_digits.cu), two rows that stand
+    for their digits by rho rho' / 10 <= 0.63 sqrt(K), 5.5 such deviations among 10^5
+    elements; and where the terms have one sign (the diagonal) the K partial sums
+    round by up to half an ulp of the value each, sqrt(K) of them in the rms, and
+    once to store."""
+    rng = np.random.default_rng(N + K)
+    b = 3.0 * rng.normal(size=(N, K))
+    d = rng.uniform(0.4, 4.0, K)
+    chi = np.stack([4 / d, 4 * d / (d * d + 1.0)])
+    g = 10.0 ** (-4 * rng.uniform(size=K))
+    if rows == "opposite":
+        b *= np.where(np.arange(N)[:, None] % 2 == 0, g, 1e-4 / g)
+    if rows == "some opposite":
+        b[100:103] *= g
+        b[257:260] *= 1e-4 / g
+    if rows == "outliers":
+        b[::5, 7] = 1e6
+        b[3::5, 900] = 1e7
+    if rows == "zeros":
+        b[[0, 100, 255]] = 0.0
+    got = p0(env, b, chi)
+    bl = b.astype(np.longdouble)
+    for w, c in enumerate(chi):
+        ref = (bl * c) @ bl.T + np.eye(N)
+        rss = np.sqrt((b * b * c * c) @ (b * b).T)
+        err = np.abs(got[w] - ref).astype(float)
+        bound = 2.0 ** -53 * (3.5 * np.sqrt(K) * rss + (1 + np.sqrt(K)) * np.abs(ref).astype(float))
+        assert (err - bound).max() <= 0
+        assert np.array_equal(got[w], got[w].T)
+    b[7, 11] = np.nan
+    bad = ~np.isfinite(p0(env, b, chi))
+    assert bad[:, 7].all() and bad[:, :, 7].all() and bad.sum() == 2 * (2 * N - 1)
