@@ -1204,12 +1204,15 @@ bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int n
   return true;
 }
 
-// C[m][n] = sum_k A[m][k] B[n][k] (16-byte aligned rows, even lda and ldb).
+// C[m][n] = sum_k A[m][k] B[n][k].  The rows are read two entries at a time:
+// operands that are not 16-byte aligned with even leading dimensions are left to
+// the caller's other path, which refuses them.
 bool gemm_nt_digits(qx_ctx* ctx, const double* A, int M, int lda, const double* B, int N, int ldb, int K, double* C,
                     int ldc) {
   // From K = 161 on (two K blocks) and a few tiles each way: below, the
   // padding and the digits cost what the faster products give.
   if (K <= 160 || K > dgt::KMAX || M < 2 * dgt::TM || N < 2 * dgt::TN) return false;
+  if (lda % 2 || ldb % 2 || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return false;
   const int ldd = round_up(K, 16);
   const size_t row = (size_t)7 * ldd, budget = digit_budget(ctx);
   const int cap = (int)std::min<size_t>(budget / row, 1u << 30) / 256 * 256;
