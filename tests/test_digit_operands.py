@@ -8,7 +8,7 @@ import pytest
 CALL = """
 import ctypes as C
 from quasix_b200 import _native
-f = _native.load()._ZN2qx14gemm_nt_digitsEP6qx_ctxPKdiiiS3_iiiPdi
+f = _native.load()._ZN2qx14gemm_nt_digitsEP6qx_ctxPKdiiS3_iiiPdi
 f.restype = C.c_bool
 a, lda, b, ldb = {args}
 i, p = C.c_int, C.c_void_p
