@@ -14,6 +14,7 @@ namespace qx {
 // Eight warps of 16 x 32: the products of a Davidson step 22.0 -> 18.7 us each
 // against four of 32 x 32.
 using GemmTile = F64Tile<64, 64, 4, 2, 3>;
+static_assert(GemmTile::BM == kRoughRows && GemmTile::BN == kRoughRows, "blocks of rho");
 
 // C[b][m][n] (or the split-K partial) = sum_{k in split} A[b][m][k] B[b][n][k]
 __global__ void __launch_bounds__(GemmTile::THREADS) k_gemm_nt(GemmNT g, double* __restrict__ part) {
@@ -21,6 +22,7 @@ __global__ void __launch_bounds__(GemmTile::THREADS) k_gemm_nt(GemmNT g, double*
   extern __shared__ double smem[];
   const int nsplit = g.splitk;
   const int b = blockIdx.z / nsplit, sk = blockIdx.z % nsplit;
+  if (g.roughA && !rough_tile(g.roughA[blockIdx.y], g.roughB[blockIdx.x], g.rough_limit)) return;
   const int m0 = blockIdx.y * T::BM, n0 = blockIdx.x * T::BN;
   const int kchunk = ((g.K + nsplit - 1) / nsplit + T::BK - 1) / T::BK * T::BK;
   const int kbeg = sk * kchunk;

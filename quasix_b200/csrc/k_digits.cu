@@ -41,6 +41,7 @@
 #include <cmath>
 
 #include "digit_rowdot.cuh"
+#include "qx_blas.cuh"
 #include "qx_internal.cuh"
 #include "tc_ptx.cuh"
 
@@ -94,8 +95,11 @@ struct DigitArgs {
   // out and ldo allow 32-byte stores).
   int lower, add, wide;
   // lower: A is the batched operand too (scaleA = scaleB).
-  const int* skip;      // nothing to do once *skip reaches skip_at (null: never)
-  int skip_at;
+  // Nothing to do when the lowest rho (as RoughRows has it) of A times that of B is
+  // above the limit.
+  const unsigned* lowA;
+  const unsigned* lowB;
+  float rough_limit;
   double* out;
   int ldo;
   size_t out_stride;
@@ -362,7 +366,7 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
     if (threadIdx.x == 0) atomicCAS(args.err, 0, 40);
     return;
   }
-  if (MODE != DIGIT_ROWDOT && args.skip && *args.skip >= args.skip_at) return;
+  if (MODE != DIGIT_ROWDOT && __uint_as_float(~*args.lowA) * __uint_as_float(~*args.lowB) > args.rough_limit) return;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + P::BAR_OFF);
@@ -845,13 +849,50 @@ __device__ __forceinline__ unsigned long long warp_max(unsigned long long m) {
   return m;
 }
 
-// What the split finds out about the rows besides their scales (either may be
+// How far fixed point suits the rows, by blocks of 64: block[w nblk + r / 64] the
+// largest rho of its rows, lowest the complement of the smallest of all (as bit
+// patterns of floats, zero on entry).
+//
+// The rounding of an entry (2^-55 of the bound 2^e) and the dropped digit products
+// make an error of a product of two rows, in 2^-53 of the root-sum-square of its
+// terms, of about rho rho' / 10, rho = 2^e / rms.  The DMMA kernel's sums of K
+// random terms make 0.28 sqrt(K).  Tiles stand for their digits up to rho rho' =
+// 6.25 sqrt(K) in P0 and 10 sqrt(K) in gemm_nt_digits (rough_limit, of the blocks'
+// largest rho: all but a few of a tile's elements lie well below), of rows that
+// share most of their large entries: a row
+// more than twice as many of whose entries have a zero top digit, |x| < 2^(e - 8),
+// as of a normal row (0.8 rho / 256 of them; weighted ones 1.3, and the margin of a
+// small K) has an infinite rho here, as one that is not finite.
+// Measured for normal B and the weights of zero frequency, digits / DMMA, rms over the
+// elements: K = 1024 4.6 / 8.5, 2020 5.5 / 12, 5270 5.9 / 19, 10 400 7.1 / 28.  In an
+// exact model, K = 10 400: an entry of 30 rms in each row 42; rows of log-uniform
+// entries over one decade, up where the other's are down, 24, over one and a half
+// (infinite, as all that follow) 73, over four 2 10^4.
+constexpr int ROUGH_ROWS = kRoughRows;
+struct RoughRows {
+  unsigned* block;
+  unsigned* lowest;
+  int nblk;
+};
+// A row's scale 2^(e - 7), sum of squares and number of zeros of its K top digits.
+__device__ __forceinline__ void mark_rough(const RoughRows& g, int w, int r, double scale, long long squares, int zeros,
+                                           int K) {
+  if (scale == 0.0) return;  // a zero row
+  const float k2 = sqrtf((float)K), rho = 128.0f * k2 / sqrtf((float)squares);
+  const bool suits = isfinite(scale) && zeros <= 0x1p-8f * 1.6f * rho * K + 0.5f * k2;
+  const unsigned bits = __float_as_uint(suits ? rho : INFINITY);
+  atomicMax(g.block + (size_t)w * g.nblk + r / ROUGH_ROWS, bits);
+  atomicMax(g.lowest, ~bits);
+}
+
+// What the split finds out about the rows besides their scales (each may be
 // null): norm[r], |row r| relative to 2^e, from above (the top digits' and their
-// rounding's); and per batch the largest 2^e and the largest |row| (as bit
-// patterns, zero on entry; a NaN is larger than all).
+// rounding's); per batch the largest 2^e and the largest |row| (as bit patterns,
+// zero on entry; a NaN is larger than all); the marked blocks of rows.
 struct SplitStats {
   double* norm;
   unsigned long long* most;  // [batch][2]
+  RoughRows rough;
 };
 
 // Sum over the TPR threads of a row (every thread of the block calls it).
@@ -905,15 +946,18 @@ __global__ void __launch_bounds__(256) k_digit_split(const double* __restrict__ 
     load8(p, k, lim, x);
     digit_store8(x, sc, d + k, slab, top);
   }
-  const double squares = (double)row_sum<TPR>(top.squares, redi);
+  const long long squares = row_sum<TPR>(top.squares, redi);
+  const long long zeros = TPR == 256 ? (__syncthreads(), row_sum<TPR>(top.zeros, redi)) : row_sum<TPR>(top.zeros, redi);
   if (live && t == 0) {
     scale[(size_t)w * lds + r] = sc.sc;
-    const double norm = (sqrt(squares) + 0.5 * sqrt((double)lim)) * 0x1p-7, bound = sc.sc * 128.0;
+    const double norm = (sqrt((double)squares) + 0.5 * sqrt((double)lim)) * 0x1p-7, bound = sc.sc * 128.0;
     if (st.norm) st.norm[r] = norm;
     if (st.most) {
       atomicMax(st.most + 2 * w, (unsigned long long)__double_as_longlong(bound));
       atomicMax(st.most + 2 * w + 1, (unsigned long long)__double_as_longlong(bound * norm));
     }
+    // (less the zeros from K to ldk)
+    if (st.rough.block) mark_rough(st.rough, w, r, sc.sc, squares, (int)zeros - (end - lim), lim);
   }
 }
 
@@ -940,36 +984,6 @@ __global__ void __launch_bounds__(256) k_digit_xt(const double* __restrict__ b, 
     const rowdot::Words w = rowdot::x_words(fin ? __double2ll_rn(v * f1 * f2) : 0);
     dst[y * 32 + tx] = make_int2(w.lo, w.hi);
   }
-}
-
-// Rows that fixed point does not suit, by blocks of 64: block[w nblk + r / 64]
-// (zero on entry) and the number of blocks marked.
-//
-// The rounding of an entry (2^-55 of the bound 2^e) and the dropped digit products
-// make an error of a product of two rows, in 2^-53 of the root-sum-square of its
-// terms, of about rho rho' / 10, rho = 2^e / rms.  The DMMA kernel's sums of K
-// random terms make 0.28 sqrt(K).  A row stands for its digits up to rho = 2.5
-// K^(1/4), and while at most twice as many of its entries have a zero top digit,
-// |x| < 2^(e - 8), as of a normal row (0.8 rho / 256 of them; weighted ones 1.3, and the
-// margin of a small K): two such rows share most of their large entries.
-// Measured for normal B and the weights of zero frequency, digits / DMMA, rms over the
-// elements: K = 1024 4.6 / 8.5, 2020 5.5 / 12, 5270 5.9 / 19, 10 400 7.1 / 28.  In an
-// exact model, K = 10 400: an entry of 30 rms in a row (marked) 42; rows of
-// log-uniform entries over one decade, up where the other's are down, 24, over one
-// and a half (marked, as all that follow) 73, over four 2 10^4.
-constexpr int ROUGH_ROWS = kRoughRows;
-struct RoughRows {
-  int* block;
-  int* count;
-  int nblk;
-};
-// A row's scale 2^(e - 7), sum of squares and number of zeros of its K top digits.
-__device__ __forceinline__ void mark_rough(const RoughRows& g, int w, int r, double scale, long long squares, int zeros,
-                                           int K) {
-  if (scale == 0.0) return;
-  const double k2 = sqrt((double)K), rho = 128.0 * k2 / sqrt((double)squares);
-  if (isfinite(scale) && rho <= 2.5 * sqrt(k2) && zeros <= 0x1p-8 * 1.6 * rho * K + 0.5 * k2) return;
-  if (atomicExch(g.block + (size_t)w * g.nblk + r / ROUGH_ROWS, 1) == 0) atomicAdd(g.count, 1);
 }
 
 // Digits of b[P][k] sqrt(chi[w][k]) for DG_R rows and DG_F frequencies per block:
@@ -1140,7 +1154,7 @@ static bool try_reserve(DevBuf& b, size_t bytes) {
 }
 
 static void split_rows(qx_ctx* ctx, const double* src, int rows, int K, int ld, size_t stride, int batch, int lower,
-                       int8_t* dig, int ldk, double* scale, int lds, SplitStats st = {nullptr, nullptr}) {
+                       int8_t* dig, int ldk, double* scale, int lds, SplitStats st = {}) {
   if (K <= 2048)
     k_digit_split<32><<<dim3(ceil_div(rows, 8), batch), 256, 0, ctx->stream>>>(src, rows, K, ld, stride, lower, dig,
                                                                              ldk, scale, lds, st);
@@ -1167,11 +1181,12 @@ bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int n
   if (!try_reserve(db, per * fc) ||
       !try_reserve(ds, (n_root + n_scale) * sizeof(double) + n_flag * sizeof(int)))
     return false;
-  // Roots of the weights; scales, the number of marked blocks and the blocks (zeroed together).
+  // Roots of the weights; scales and the rows' rho (zeroed together).
   double* root = ds.as<double>();
   double* sb = root + n_root;
-  int* marked = reinterpret_cast<int*>(sb + n_scale);
-  const RoughRows rough{marked + 1, marked, nblk};
+  unsigned* marks = reinterpret_cast<unsigned*>(sb + n_scale);
+  const RoughRows rough{marks + 1, marks, nblk};
+  const float limit = 6.25f * std::sqrt((float)nov);
   for (int w0 = 0; w0 < nw; w0 += fc) {
     const int n = std::min(fc, nw - w0);
     QX_CUDA(cudaMemsetAsync(sb, 0, n_scale * sizeof(double) + n_flag * sizeof(int), ctx->stream));
@@ -1190,16 +1205,16 @@ bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int n
     a.out = eps + (size_t)w0 * eps_stride;
     a.ldo = ldn;
     a.out_stride = eps_stride;
-    a.skip = marked;
-    a.skip_at = nblk * n;
+    a.lowA = a.lowB = rough.lowest;
+    a.rough_limit = limit;
     for (int k0 = 0; k0 < nov; k0 += dgt::KMAX) {
       a.K = std::min(dgt::KMAX, nov - k0);
       a.add = k0 > 0;
       launch_digit_gemm<DIGIT_LOWER>(ctx, db.as<int8_t>() + k0, ldk, db.as<int8_t>() + k0, ldk, a);
     }
-    // The tiles with marked rows by the DMMA kernel.
+    // The tiles above the limit by the DMMA kernel.
     launch_eps_dmma(ctx, bov, ldov, naux, nov, chi + (size_t)w0 * ldov, n, eps + (size_t)w0 * eps_stride, ldn,
-                    eps_stride, rough.block);
+                    eps_stride, rough.block, limit);
   }
   return true;
 }
@@ -1217,20 +1232,27 @@ bool gemm_nt_digits(qx_ctx* ctx, const double* A, int M, int lda, const double* 
   const size_t row = (size_t)7 * ldd, budget = digit_budget(ctx);
   const int cap = (int)std::min<size_t>(budget / row, 1u << 30) / 256 * 256;
   const int mc = std::min(M, std::max(256, cap)), nc = std::min(N, std::max(256, cap));
-  const int lds = round_up(nc, dgt::TN);
+  const int lds = round_up(nc, dgt::TN), blkA = ceil_div(mc, ROUGH_ROWS), blkB = ceil_div(nc, ROUGH_ROWS);
   DevBuf &da = ctx->ws[WS_DIG_A], &db = ctx->ws[WS_DIG_B], &ds = ctx->ws[WS_DIG_S];
-  if (!try_reserve(da, row * mc) || !try_reserve(db, row * nc) ||
-      !try_reserve(ds, ((size_t)mc + lds) * sizeof(double)))
-    return false;
+  const size_t b_bytes = lds * sizeof(double) + (size_t)round_up(blkB + 1, 2) * sizeof(int);
+  const size_t a_bytes = mc * sizeof(double) + (size_t)(blkA + 1) * sizeof(int);
+  if (!try_reserve(da, row * mc) || !try_reserve(db, row * nc) || !try_reserve(ds, b_bytes + a_bytes)) return false;
+  // Scales of B and its rows' rho; the same of A.
   double* sb = ds.as<double>();
-  double* sa = sb + lds;
-  QX_CUDA(cudaMemsetAsync(sb, 0, (size_t)lds * sizeof(double), ctx->stream));
+  unsigned* mb = reinterpret_cast<unsigned*>(sb + lds);
+  double* sa = reinterpret_cast<double*>(ds.as<char>() + b_bytes);
+  unsigned* ma = reinterpret_cast<unsigned*>(sa + mc);
+  const RoughRows ra{ma + 1, ma, blkA}, rb{mb + 1, mb, blkB};
   for (int n0 = 0; n0 < N; n0 += nc) {
     const int n = std::min(nc, N - n0);
-    split_rows(ctx, B + (size_t)n0 * ldb, n, K, ldb, 0, 1, 0, db.as<int8_t>(), ldd, sb, lds);
+    QX_CUDA(cudaMemsetAsync(sb, 0, b_bytes, ctx->stream));
+    split_rows(ctx, B + (size_t)n0 * ldb, n, K, ldb, 0, 1, 0, db.as<int8_t>(), ldd, sb, lds, {nullptr, nullptr, rb});
     for (int m0 = 0; m0 < M; m0 += mc) {
       const int m = std::min(mc, M - m0);
-      if (n0 == 0 || mc < M) split_rows(ctx, A + (size_t)m0 * lda, m, K, lda, 0, 1, 0, da.as<int8_t>(), ldd, sa, 0);
+      if (n0 == 0 || mc < M) {
+        QX_CUDA(cudaMemsetAsync(ma, 0, (size_t)(blkA + 1) * sizeof(int), ctx->stream));
+        split_rows(ctx, A + (size_t)m0 * lda, m, K, lda, 0, 1, 0, da.as<int8_t>(), ldd, sa, 0, {nullptr, nullptr, ra});
+      }
       DigitArgs a{};
       a.M = m;
       a.N = n;
@@ -1242,7 +1264,32 @@ bool gemm_nt_digits(qx_ctx* ctx, const double* A, int M, int lda, const double* 
       a.out = C + (size_t)m0 * ldc + n0;
       a.ldo = ldc;
       a.wide = ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 31) == 0;
+      a.lowA = ma;
+      a.lowB = mb;
+      // The adjoint's rows of G have a large diagonal (rho 5 to 20): a matrix X X^T of
+      // 400 columns times normal rows, K = 700, err by 10 (the DMMA's sums by 8.6, in
+      // 2^-53 of the root-sum-square), its elements of rho rho' = 6 to 10 sqrt(K), 4 %
+      // of them, by 19.  The gradient's error is the same either way (1.2 to 1.6 e-15).
+      a.rough_limit = 10.0f * std::sqrt((float)K);
       launch_digit_gemm<DIGIT_PLAIN>(ctx, da.as<int8_t>(), ldd, db.as<int8_t>(), ldd, a);
+      // The tiles above the limit by the DMMA kernel.
+      GemmNT g{};
+      g.M = m;
+      g.N = n;
+      g.K = K;
+      g.A = A + (size_t)m0 * lda;
+      g.lda = lda;
+      g.B = B + (size_t)n0 * ldb;
+      g.ldb = ldb;
+      g.C = a.out;
+      g.ldc = ldc;
+      g.batch = 1;
+      g.alpha = 1.0;
+      g.splitk = 1;
+      g.roughA = ra.block;
+      g.roughB = rb.block;
+      g.rough_limit = a.rough_limit;
+      gemm_nt_f64(ctx, g);
     }
   }
   return true;
@@ -1274,7 +1321,7 @@ bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int np
   int* redo = reinterpret_cast<int*>(norm + pc);
   for (int p0 = 0; p0 < npair; p0 += pc) {
     const int np = std::min(pc, npair - p0);
-    split_rows(ctx, bpt + (size_t)p0 * ldk, np, naux, ldk, 0, 1, 0, da.as<int8_t>(), ldd, sa, 0, {norm, nullptr});
+    split_rows(ctx, bpt + (size_t)p0 * ldk, np, naux, ldk, 0, 1, 0, da.as<int8_t>(), ldd, sa, 0, {norm, nullptr, {}});
     k_digit_xt<<<dim3(lds / 32, ceil_div(np, 32)), 256, 0, ctx->stream>>>(bpt + (size_t)p0 * ldk, np, naux, ldk, sa, lds,
                                                                            xt);
     check_launch(ctx);
@@ -1283,7 +1330,7 @@ bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int np
       if (p0 == 0 || fc < nw) {
         QX_CUDA(cudaMemsetAsync(sb, 0, ((size_t)(lds + 2) * fc + 1) * sizeof(double), ctx->stream));
         split_rows(ctx, wc + (size_t)w0 * wc_stride, naux, naux, ldn, wc_stride, n, 1, db.as<int8_t>(), ldd, sb, lds,
-                   {nullptr, most});
+                   {nullptr, most, {}});
       } else {
         QX_CUDA(cudaMemsetAsync(redo_count, 0, sizeof(int), ctx->stream));
       }

@@ -46,12 +46,13 @@ void launch_chi(qx_ctx* ctx, const double* energies, int nocc, int nvir, const d
 // Eight warps of 16 x 32 (four of 32 x 32 left the FP64 tensor pipe waiting on
 // its operands: 22.5 us at naux 139 / nov 352, now 18.1; a batch 658 -> 572 us).
 using EpsTile = F64Tile<64, 64, 4, 2, 3>;
-static_assert(EpsTile::BM == kRoughRows && EpsTile::BN == kRoughRows, "blocks of marked rows");
+static_assert(EpsTile::BM == kRoughRows && EpsTile::BN == kRoughRows, "blocks of rho");
 
 __global__ void __launch_bounds__(EpsTile::THREADS) k_eps_f64(const double* __restrict__ bov, int ldov, int naux,
                                                               int nov, const double* __restrict__ chi,
                                                               double* __restrict__ eps, int ldn,
-                                                              size_t eps_stride, const int* __restrict__ rough) {
+                                                              size_t eps_stride, const unsigned* __restrict__ rough,
+                                                              float rough_limit) {
   using T = EpsTile;
   extern __shared__ double smem[];
   // Lower-triangular tile index -> (tm, tn), tm >= tn.
@@ -63,8 +64,8 @@ __global__ void __launch_bounds__(EpsTile::THREADS) k_eps_f64(const double* __re
   const int w = blockIdx.y;
   const int m0 = tm * T::BM, n0 = tn * T::BN;
   if (rough) {
-    const int* g = rough + (size_t)w * ((naux + T::BM - 1) / T::BM);
-    if (!(g[tm] | g[tn])) return;
+    const unsigned* g = rough + (size_t)w * ((naux + T::BM - 1) / T::BM);
+    if (!rough_tile(g[tm], g[tn], rough_limit)) return;
   }
   double acc[T::MI][T::NJ][2];
 #pragma unroll
@@ -100,11 +101,11 @@ void launch_eps_fp64(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov
   if (smooth && naux >= 256 && nov >= 1024 &&
       launch_eps_digits(ctx, bov, ldov, naux, nov, chi, nw, eps, ldn, eps_stride))
     return;
-  launch_eps_dmma(ctx, bov, ldov, naux, nov, chi, nw, eps, ldn, eps_stride, nullptr);
+  launch_eps_dmma(ctx, bov, ldov, naux, nov, chi, nw, eps, ldn, eps_stride, nullptr, 0.0f);
 }
 
 void launch_eps_dmma(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw, double* eps,
-                     int ldn, size_t eps_stride, const int* rough) {
+                     int ldn, size_t eps_stride, const unsigned* rough, float rough_limit) {
   using T = EpsTile;
   const int tiles = ceil_div(naux, T::BM);
   dim3 grid(tiles * (tiles + 1) / 2, nw);
@@ -112,7 +113,8 @@ void launch_eps_dmma(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov
   attr_once(ctx->device, [&] {
     QX_CUDA(cudaFuncSetAttribute(k_eps_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM));
   });
-  k_eps_f64<<<grid, T::THREADS, T::SMEM, ctx->stream>>>(bov, ldov, naux, nov, chi, eps, ldn, eps_stride, rough);
+  k_eps_f64<<<grid, T::THREADS, T::SMEM, ctx->stream>>>(bov, ldov, naux, nov, chi, eps, ldn, eps_stride, rough,
+                                                             rough_limit);
   check_launch(ctx);
 }
 

@@ -22,6 +22,11 @@ struct GemmNT {
   int batch;
   double alpha, beta;
   int splitk;
+  // When given (splitk 1): only the tiles where the product of the blocks' rho (bit
+  // patterns, roughA[m / kRoughRows] and roughB[n / kRoughRows]) is above rough_limit.
+  const unsigned* roughA;
+  const unsigned* roughB;
+  float rough_limit;
 };
 void gemm_nt_f64(qx_ctx* ctx, GemmNT g);
 

@@ -262,11 +262,16 @@ bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int n
                        double* eps, int ldn, size_t eps_stride);
 bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc,
                                  int ldn, size_t wc_stride, int nw, double* v, int ldv);
-// P0 by the DMMA kernel; rough (or null): only the tiles with a marked block of
-// kRoughRows rows, rough[w ceil(naux / kRoughRows) + block].
+// How far fixed point suits rows, by blocks of kRoughRows (k_digits.cu: rho, as the bit
+// pattern of a float; infinite rows times zero rows count as above any limit).
 constexpr int kRoughRows = 64;
+__device__ __forceinline__ bool rough_tile(unsigned a, unsigned b, float limit) {
+  return !(__uint_as_float(a) * __uint_as_float(b) <= limit);
+}
+// P0 by the DMMA kernel; rough (or null): only the tiles where the product of the
+// blocks' rho, rough[w ceil(naux / kRoughRows) + block], is above the limit.
 void launch_eps_dmma(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw, double* eps,
-                     int ldn, size_t eps_stride, const int* rough);
+                     int ldn, size_t eps_stride, const unsigned* rough, float rough_limit);
 // The DMMA contraction of the listed blocks of kPairRedoRows pairs (device list and
 // count), which the digits may not hold.
 constexpr int kPairRedoRows = 64;

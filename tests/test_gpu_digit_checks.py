@@ -12,6 +12,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+GEMM = "_ZN2qx14gemm_nt_digitsEP6qx_ctxPKdiiS3_iiiPdi"
 P0 = "_ZN2qx15launch_eps_fp64EP6qx_ctxPKdiiiS3_iPdimi"
 CONTRACT = "_ZN2qx25launch_pair_contract_fp64EP6qx_ctxPKdiiiS3_imiPdi"
 
@@ -154,3 +155,41 @@ def test_p0_of_rough_rows(env, N, K, rows):
     b[7, 11] = np.nan
     bad = ~np.isfinite(p0(env, b, chi))
     assert bad[:, 7].all() and bad[:, :, 7].all() and bad.sum() == 2 * (2 * N - 1)
+
+
+@pytest.mark.parametrize("M,N,K,rows", [(256, 256, 161, "normal"), (300, 259, 170, "some opposite"),
+                                        (257, 400, 301, "opposite"), (500, 256, 700, "outliers"),
+                                        (256, 321, 200, "zeros")])
+def test_product_of_rough_rows(env, M, N, K, rows):
+    """C = A B^T with the rows of test_p0_of_rough_rows; tiles that stand for their
+    digits err by up to sqrt(K) (5.5 such deviations)."""
+    torch, ctx = env
+    rng = np.random.default_rng(M + K)
+    a, b = rng.normal(size=(M, K)), rng.normal(size=(N, K))
+    g = 10.0 ** (-4 * rng.uniform(size=K))
+    if rows == "opposite":
+        a, b = a * g, b * 1e-4 / g
+    if rows == "some opposite":
+        a[100:103] *= g
+        b[257:] *= 1e-4 / g
+    if rows == "outliers":
+        a[::70, 7] = 1e6
+        b[3, 90] = 1e7
+    if rows == "zeros":
+        a[[0, 100, 255]] = 0.0
+        b[320] = 0.0
+    ld, ldc = (K + 7) // 8 * 8, N + 3
+    ta, tb = (torch.from_numpy(_pad(x, ld)).cuda() for x in (a, b))
+    c = torch.full((M, ldc), 7.0, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    f = getattr(ctx.lib, GEMM)
+    f.restype = C.c_bool
+    assert f(ctx.handle, _ptr(ta), C.c_int(M), C.c_int(ld), _ptr(tb), C.c_int(N), C.c_int(ld), C.c_int(K), _ptr(c),
+             C.c_int(ldc))
+    torch.cuda.synchronize()
+    got = c.cpu().numpy()
+    assert (got[:, N:] == 7.0).all()
+    ref = a.astype(np.longdouble) @ b.astype(np.longdouble).T
+    rss = np.sqrt((a * a) @ (b * b).T)
+    bound = 2.0 ** -53 * (5.5 * np.sqrt(K) * rss + (1 + np.sqrt(K)) * np.abs(ref).astype(float))
+    assert (np.abs(got[:, :N] - ref).astype(float) - bound).max() <= 0
