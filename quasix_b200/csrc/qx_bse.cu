@@ -398,11 +398,9 @@ struct qx_bse {
   DevArr kd_split, kd_scale;
   int ldg = 0;
   bool kd = false;
-  // FP64: the contracted direct kernel C[(i,j)][(a,b)], formed when it pays and
-  // fits (ensure_kd_f64), and the vectors applied so far.
+  // FP64, for the length of a solve: the contracted direct kernel C[(i,j)][(a,b)],
+  // when it pays and fits (form_kd_f64).
   DevArr kd_f64;
-  bool kd_f64_tried = false;
-  long long applied = 0;
   DevArr x_split;                    // split forms: hi/lo of the packed vectors
   DevArr xp, T, Yd, Z, Yx, Xr, Yr;  // matvec scratch
   DevArr gTt, gTp, gTpT, gdijT, gM, gG1, gG, gU;  // root-gradient scratch
@@ -517,21 +515,22 @@ static void kd_apply(qx_bse* B, const double* X, int nvec) {
 // contracted once).  The factored direct term costs 4 nov nvir naux FLOPs per
 // vector each time, C's one product 2 nov^2 naux FLOPs once, four times faster
 // as one product of digits: as much as nocc / 8 vectors with digits, nocc / 2
-// without.  It is formed when that many vectors have been applied the factored
-// way, so that no run of calls costs more than twice the better form; a solve of
-// n roots counts 8 n vectors ahead (it takes 10 to 100 per root).
-// Dimension 10 400, naux 1000, ten vectors: 3.1 ms factored, 0.6 ms contracted,
-// 2.5 ms to form it; dimension 3264, naux 560, five vectors: 190 and 60 us, 0.4 ms.
+// without.  A solve of n roots applies 10 n to 100 n vectors: it forms C when 8 n
+// pay for it, at its start, and gives the memory back at its end.  So a call
+// depends on its own arguments only: the factored form is what apply uses, before
+// and after solves.
+// Whole solves for 1, 3 and 10 roots, factored and contracted, allocation
+// included: dimension 1280 32.6, 68.6, 118 and 30.2, 67.2, 116 ms; 3264 80, 143, 242 and
+// 72, 127, 178 ms; 10 400 336, 471, 977 and 280, 320, 458 ms; 26 400 0.91, 2.0, 5.7 and 0.64,
+// 0.74, 1.05 s.  Ten vectors at dimension 10 400 take 3.1 ms factored, 0.6 ms contracted.
 // Held when its nov^2 doubles take at most 16 GB, the bound of the split forms'
-// K^d, and at most half of the free memory; else, and below dimension 512, where
-// both are a few launches, the factored form stays.
-static void ensure_kd_f64(qx_bse* B, long long vectors) {
-  if (B->precision != QX_PREC_FP64 || B->kd_f64_tried) return;
-  if (vectors * (B->naux > 160 ? 8 : 2) < B->nocc) return;
-  B->kd_f64_tried = true;
+// K^d, and at most half of the free memory; else, and below dimension 1024 (at 512 a
+// solve of 12 to 36 ms took 0.5 ms longer with it), the factored form stays.
+static void form_kd_f64(qx_bse* B, int n_roots) {
+  if (B->precision != QX_PREC_FP64 || 8ll * n_roots * (B->naux > 160 ? 8 : 2) < B->nocc) return;
   qx_ctx* ctx = B->ctx;
   const size_t n2 = (size_t)B->nov * B->nov;
-  if (B->nov < 512 || n2 * sizeof(double) > ((size_t)16 << 30)) return;
+  if (B->nov < 1024 || n2 * sizeof(double) > ((size_t)16 << 30)) return;
   // dabT [a][Q][b] back to [a][b][Q], some virtuals a at a time.
   const size_t slab = (size_t)B->nvir * B->ldq;
   const int na = (int)std::max<size_t>(1, std::min<size_t>(B->nvir, ((size_t)64 << 20) / (slab * sizeof(double))));
@@ -581,10 +580,6 @@ static void ensure_kd_f64(qx_bse* B, long long vectors) {
 static void bse_apply_rows(qx_bse* B, const double* X, double* Y, int nvec, bool need_T = false) {
   qx_ctx* ctx = B->ctx;
   const int nocc = B->nocc, nvir = B->nvir, naux = B->naux;
-  if (!need_T) {
-    ensure_kd_f64(B, B->applied);
-    B->applied += nvec;
-  }
   B->Yd.alloc((size_t)nocc * nvir * nvec);
   if (B->kd_f64.p && !need_T) {
     kd_apply(B, X, nvec);
@@ -1151,7 +1146,11 @@ qx_status qx_bse_davidson(qx_bse* B, const qx_davidson_config* cfgp, double* eig
                           int* converged_out, double* residual_norms, int* iterations) {
   if (!B || !cfgp) return QX_ERR_INVALID_INPUT;
   return bse_guard(B->ctx, [&] {
-    ensure_kd_f64(B, B->applied + 8ll * std::max(1, cfgp->n_roots));
+    struct Contracted {  // for this solve
+      qx_bse* B;
+      ~Contracted() { B->kd_f64.free(); }
+    } contracted{B};
+    form_kd_f64(B, cfgp->n_roots);
     davidson_run(B->ctx, B->dav, B->nov, B->ldov, B->delta.p, B->h_delta,
                  [&](const double* x, double* y, int count) { bse_apply_rows(B, x, y, count); }, *cfgp, eigenvalues,
                  eigenvectors, converged_out, residual_norms, iterations);
