@@ -83,6 +83,13 @@ qx_status qx_ctx_set_p0_form(qx_ctx* ctx, int form);
  * QX_CONTRACT_AUTO (default) takes the pair form. */
 enum { QX_CONTRACT_AUTO = 0, QX_CONTRACT_SINGLE = 1, QX_CONTRACT_PAIR = 2 };
 qx_status qx_ctx_set_contraction_form(qx_ctx* ctx, int form);
+/* Device memory that the context may hold for the operands of the FP64
+ * contractions on the integer tensor pipe (no reference counterpart), in bytes;
+ * 0 (default): up to 4 GiB, for each worker of a batch 1.25 GiB, and one frequency
+ * and 256 rows in any case.  Problems that need more run in chunks, with the same
+ * results; a product whose smallest chunk does not fit a given limit runs on the
+ * FP64 tensor pipe.  The workers of a batch share a given limit in equal parts. */
+qx_status qx_ctx_set_digit_workspace(qx_ctx* ctx, size_t bytes);
 /* Library version string. */
 const char* qx_version(void);
 

@@ -97,6 +97,7 @@ SIGNATURES = {
     "qx_ctx_last_guard_stats": (C.c_int, [_vp, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]),
     "qx_ctx_set_p0_form": (C.c_int, [_vp, C.c_int]),
     "qx_ctx_set_contraction_form": (C.c_int, [_vp, C.c_int]),
+    "qx_ctx_set_digit_workspace": (C.c_int, [_vp, C.c_size_t]),
     "qx_version": (C.c_char_p, []),
     "qx_get_scaled_legendre_roots": (C.c_int, [C.c_int, C.c_double, _vp, _vp]),
     "qx_get_rho_response": (C.c_int, [_vp, C.c_int, _vp, _vp, _vp, C.c_int, C.c_int, C.c_int, C.c_int, _vp]),
@@ -216,6 +217,11 @@ class Context:
     def set_contraction_form(self, form: str):
         """'auto', 'single' or 'pair' (qx_ctx_set_contraction_form)."""
         self.check(self.lib.qx_ctx_set_contraction_form(self.handle, CONTRACTION_FORM[form]))
+
+    def set_digit_workspace(self, bytes: int):
+        """Device memory for the operands of the FP64 contractions, 0 for the
+        default (qx_ctx_set_digit_workspace)."""
+        self.check(self.lib.qx_ctx_set_digit_workspace(self.handle, bytes))
 
     def guard_stats(self):
         """(guarded, reinverted): eps inversions of the last call that ran

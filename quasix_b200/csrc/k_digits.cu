@@ -1164,23 +1164,86 @@ static void split_rows(qx_ctx* ctx, const double* src, int rows, int K, int ld, 
   check_launch(ctx);
 }
 
-// Workspace for the digits of the batched operand (all frequencies of one
-// launch); larger problems run in chunks.  Batch workers share the device.
-static size_t digit_budget(qx_ctx* ctx) { return ctx->worker ? (size_t)512 << 20 : (size_t)1536 << 20; }
+// ---------------------------------------------------------------------------
+// Workspace.  A context holds at most its limit over the four slots: 3/8 for the
+// batched operand's digits (WS_DIG_B), 1/4 for the other's (WS_DIG_A), 3/8 for the
+// rest (scales, the pairs' integers and partial sums).  Larger problems run in
+// chunks.  By default one frequency and 256 rows are always taken; within a limit
+// that the caller has set, a product whose smallest chunk does not fit takes the
+// DMMA kernels.  Chunks do not change a result: frequencies and rows are
+// independent.
+// ---------------------------------------------------------------------------
+// 4 GB: P0 at nmo 300 / naux 1000 / 32 frequencies takes two chunks, its contraction of
+// all pairs one.  Batch workers share the device: 1.25 GB.
+size_t digit_limit(const qx_ctx* ctx) {
+  return ctx->digit_limit ? ctx->digit_limit : ctx->worker ? (size_t)1280 << 20 : (size_t)4096 << 20;
+}
+struct DigitPlan {
+  int fc = 0, rows = 0;       // frequencies and rows (pairs, or of A) per chunk; none: 0
+  size_t a = 0, b = 0, s = 0, p = 0;  // bytes of the slots
+};
+
+static DigitPlan plan_p0(int naux, int nov, int ldov, int nw, size_t limit, bool strict) {
+  DigitPlan d;
+  const int ldk = round_up(nov, 16), lds = round_up(naux, dgt::TN), nblk = ceil_div(naux, ROUGH_ROWS);
+  const size_t per = (size_t)7 * naux * ldk, per_s = ((size_t)lds + ldov + nblk) * sizeof(double);
+  size_t f = std::min(limit / 8 * 3 / per, limit / 8 * 3 / per_s);
+  if (f == 0 && strict) return d;
+  f = std::max<size_t>(1, std::min<size_t>(f, nw));
+  d.fc = ceil_div(nw, ceil_div(nw, (int)f));
+  d.b = per * d.fc;
+  d.s = per_s * d.fc + 64;
+  return d;
+}
+
+static DigitPlan plan_contract(int npair, int naux, int nw, size_t limit, bool strict) {
+  DigitPlan d;
+  const int lds = round_up(naux, dgt::TN), NT = lds / dgt::TN;
+  const size_t row = (size_t)7 * round_up(naux, 16), third = limit / 8 * 3;
+  size_t f = third / (row * naux);
+  if (f == 0 && strict) return d;
+  d.fc = (int)std::max<size_t>(1, std::min<size_t>(f, nw));
+  // Per pair: digits; partial sums, integers, scale, norm and list entries.
+  const size_t per_p = ((size_t)2 * NT * d.fc + lds) * sizeof(double);
+  const size_t fixed_s = ((size_t)(lds + 2) * d.fc + 2) * sizeof(double);
+  const size_t per_s = 2 * sizeof(double) + (size_t)ceil_div(d.fc, REDO_ROWS / (int)sizeof(int));
+  size_t r = fixed_s < third ? std::min(limit / 4 / row, (third - fixed_s) / (per_p + per_s)) / 256 * 256 : 0;
+  if (r == 0 && strict && npair > 0) {
+    d.fc = 0;
+    return d;
+  }
+  r = std::max<size_t>(256, r);
+  d.rows = (int)std::min<size_t>(r, npair);
+  const size_t padded = round_up(d.rows, 256);
+  d.a = row * d.rows;
+  d.b = row * naux * d.fc;
+  d.p = ((size_t)2 * NT * d.fc * d.rows + padded * lds) * sizeof(double);
+  d.s = fixed_s + (size_t)2 * d.rows * sizeof(double) + (size_t)ceil_div(d.rows, REDO_ROWS) * d.fc * sizeof(int);
+  return d;
+}
+
+size_t digit_workspace_bytes(int naux, int nov, int npair, int nw, size_t limit) {
+  const int ldov = round_up(nov, 8);
+  const DigitPlan p0 = digits_for_p0(naux, nov) ? plan_p0(naux, nov, ldov, nw, limit, false) : DigitPlan{};
+  const DigitPlan pc = digits_for_contraction(naux) ? plan_contract(npair, naux, nw, limit, false) : DigitPlan{};
+  return std::max(p0.b, pc.b) + std::max(p0.s, pc.s) + pc.a + pc.p;
+}
+
+// From where the integer tensor pipe is the faster one: with 24 frequencies P0 took
+// 137 (DMMA) and 152 us (digits) at naux 300 / nov 949, 295 and 209 us at 350 / 1411, 474
+// and 264 us at 423 / 2020.  From K = 1024 on its error is half the DMMA's or less.
+bool digits_for_p0(int naux, int nov) { return naux >= 256 && nov >= 1024; }
 
 // eps[w] = I + B_ov diag(chi'[w]) B_ov^T, chi' >= 0.
 bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw,
                        double* eps, int ldn, size_t eps_stride) {
-  const int ldk = round_up(nov, 16);
-  const size_t per = (size_t)7 * naux * ldk;
-  const int fmax = (int)std::max<size_t>(1, std::min<size_t>(nw, digit_budget(ctx) / per));
-  const int chunks = ceil_div(nw, fmax), fc = ceil_div(nw, chunks);
+  const DigitPlan plan = plan_p0(naux, nov, ldov, nw, digit_limit(ctx), ctx->digit_limit != 0);
+  if (!plan.fc) return false;
+  const int ldk = round_up(nov, 16), fc = plan.fc;
   DevBuf &db = ctx->ws[WS_DIG_B], &ds = ctx->ws[WS_DIG_S];
   const int lds = round_up(naux, dgt::TN), nblk = ceil_div(naux, ROUGH_ROWS);
   const size_t n_scale = (size_t)lds * fc, n_flag = (size_t)nblk * fc + 1, n_root = (size_t)ldov * fc;
-  if (!try_reserve(db, per * fc) ||
-      !try_reserve(ds, (n_root + n_scale) * sizeof(double) + n_flag * sizeof(int)))
-    return false;
+  if (!try_reserve(db, plan.b) || !try_reserve(ds, plan.s)) return false;
   // Roots of the weights; scales and the rows' rho (zeroed together).
   double* root = ds.as<double>();
   double* sb = root + n_root;
@@ -1229,9 +1292,11 @@ bool gemm_nt_digits(qx_ctx* ctx, const double* A, int M, int lda, const double* 
   if (K <= 160 || K > dgt::KMAX || M < 2 * dgt::TM || N < 2 * dgt::TN) return false;
   if (lda % 2 || ldb % 2 || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return false;
   const int ldd = round_up(K, 16);
-  const size_t row = (size_t)7 * ldd, budget = digit_budget(ctx);
-  const int cap = (int)std::min<size_t>(budget / row, 1u << 30) / 256 * 256;
-  const int mc = std::min(M, std::max(256, cap)), nc = std::min(N, std::max(256, cap));
+  const size_t row = (size_t)7 * ldd, limit = digit_limit(ctx);
+  const int rows_a = (int)std::min<size_t>(limit / 4 / row, 1u << 30) / 256 * 256;
+  const int rows_b = (int)std::min<size_t>(limit / 8 * 3 / row, 1u << 30) / 256 * 256;
+  if (ctx->digit_limit && (rows_a == 0 || rows_b == 0)) return false;
+  const int mc = std::min(M, std::max(256, rows_a)), nc = std::min(N, std::max(256, rows_b));
   const int lds = round_up(nc, dgt::TN), blkA = ceil_div(mc, ROUGH_ROWS), blkB = ceil_div(nc, ROUGH_ROWS);
   DevBuf &da = ctx->ws[WS_DIG_A], &db = ctx->ws[WS_DIG_B], &ds = ctx->ws[WS_DIG_S];
   const size_t b_bytes = lds * sizeof(double) + (size_t)round_up(blkB + 1, 2) * sizeof(int);
@@ -1295,20 +1360,23 @@ bool gemm_nt_digits(qx_ctx* ctx, const double* A, int M, int lda, const double* 
   return true;
 }
 
+// The integer tensor pipe above one column tile: with 24 frequencies the
+// contraction took 44 (DMMA) and 32 us (digits) at naux 139 with 160 pairs, 72 and 35
+// us at naux 196 with 224, 178 and 84 us with 3136; at naux 86 the DMMA kernel was the
+// faster one (24 against 27 us).  Its five launches more cost ~15 us on the host, so
+// the line is drawn at 160.
+bool digits_for_contraction(int naux) { return naux > 160 && naux <= dgt::KMAX; }
+
 // v[w][p] = Bpt[p]^T Wc[w] Bpt[p] from W' (half-lower Wc).
 bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc,
                                  int ldn, size_t wc_stride, int nw, double* v, int ldv) {
-  if (naux > dgt::KMAX) return false;
-  const int ldd = round_up(naux, 16), NT = ceil_div(naux, dgt::TN);
-  const size_t row = (size_t)7 * ldd, budget = digit_budget(ctx);
-  const int fc = (int)std::max<size_t>(1, std::min<size_t>(nw, budget / (row * naux)));
-  int pc = (int)std::max<size_t>(256, std::min<size_t>(npair, budget / row));
-  pc = std::min(round_up(pc, 256), npair);
-  const int lds = NT * dgt::TN, redo_cap = ceil_div(pc, REDO_ROWS) * fc;
+  const DigitPlan plan = plan_contract(npair, naux, nw, digit_limit(ctx), ctx->digit_limit != 0);
+  if (!plan.fc) return false;
+  const int ldd = round_up(naux, 16), NT = ceil_div(naux, dgt::TN), fc = plan.fc, pc = plan.rows;
+  const size_t row = (size_t)7 * ldd;
+  const int lds = NT * dgt::TN;
   DevBuf &da = ctx->ws[WS_DIG_A], &db = ctx->ws[WS_DIG_B], &ds = ctx->ws[WS_DIG_S], &dp = ctx->ws[WS_DIG_P];
-  if (!try_reserve(da, row * pc) || !try_reserve(db, row * naux * fc) ||
-      !try_reserve(ds, ((size_t)2 * pc + (size_t)(lds + 2) * fc + 1) * sizeof(double) + redo_cap * sizeof(int)) ||
-      !try_reserve(dp, ((size_t)2 * NT * fc * pc + (size_t)round_up(pc, 256) * lds) * sizeof(double)))
+  if (!try_reserve(da, plan.a) || !try_reserve(db, plan.b) || !try_reserve(ds, plan.s) || !try_reserve(dp, plan.p))
     return false;
   int2* xt = reinterpret_cast<int2*>(dp.as<double>() + (size_t)2 * NT * fc * pc);
   // Scales of W', its largest bounds and norms, the count of the blocks to form

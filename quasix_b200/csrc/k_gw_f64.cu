@@ -92,13 +92,9 @@ __global__ void __launch_bounds__(EpsTile::THREADS) k_eps_f64(const double* __re
 
 void launch_eps_fp64(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw,
                      double* eps, int ldn, size_t eps_stride, int smooth) {
-  // The integer tensor pipe from where it is the faster one: with 24
-  // frequencies P0 took 137 (DMMA) and 152 us (digits) at naux 300 / nov 949,
-  // 295 and 209 us at 350 / 1411, 474 and 264 us at 423 / 2020.  Only for positive
-  // weights that do not differ too much (smooth); from K = 1024 on its error is
-  // half the DMMA's or less, and rows that fixed point does not suit come back
-  // here (k_digits.cu has both figures).
-  if (smooth && naux >= 256 && nov >= 1024 &&
+  // On the integer tensor pipe only for positive weights that do not differ too
+  // much (smooth); rows that fixed point does not suit come back here.
+  if (smooth && digits_for_p0(naux, nov) &&
       launch_eps_digits(ctx, bov, ldov, naux, nov, chi, nw, eps, ldn, eps_stride))
     return;
   launch_eps_dmma(ctx, bov, ldov, naux, nov, chi, nw, eps, ldn, eps_stride, nullptr, 0.0f);
@@ -1372,12 +1368,8 @@ void launch_pair_contract_redo(qx_ctx* ctx, const double* bpt, int ldk, int npai
 
 void launch_pair_contract_fp64(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc,
                                int ldn, size_t wc_stride, int nw, double* v, int ldv) {
-  // The integer tensor pipe above one column tile: with 24 frequencies the
-  // contraction took 44 (DMMA) and 32 us (digits) at naux 139 with 160 pairs,
-  // 72 and 35 us at naux 196 with 224, 178 and 84 us with 3136; at naux 86 the
-  // DMMA kernel was the faster one (24 against 27 us).  Its four launches more
-  // cost ~12 us on the host, so the line is drawn at 160.
-  if (naux > 160 && launch_pair_contract_digits(ctx, bpt, ldk, npair, naux, wc, ldn, wc_stride, nw, v, ldv))
+  if (digits_for_contraction(naux) &&
+      launch_pair_contract_digits(ctx, bpt, ldk, npair, naux, wc, ldn, wc_stride, nw, v, ldv))
     return;
   using T = PairTile;
   pair_attributes_once(ctx->device);

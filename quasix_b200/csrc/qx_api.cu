@@ -612,6 +612,18 @@ qx_status qx_ctx_set_contraction_form(qx_ctx* c, int form) {
   return QX_OK;
 }
 
+qx_status qx_ctx_set_digit_workspace(qx_ctx* c, size_t bytes) {
+  if (!c) return QX_ERR_INVALID_INPUT;
+  c->digit_limit = bytes;
+  // What a former limit allowed goes back now.
+  cudaSetDevice(c->device);
+  for (int i = WS_DIG_A; i <= WS_DIG_P; ++i) {
+    c->ws[i].release();
+    for (qx_ctx* w : c->workers) w->ws[i].release();
+  }
+  return QX_OK;
+}
+
 qx_status qx_ctx_set_p0_form(qx_ctx* c, int form) {
   if (!c || form < QX_P0_AUTO || form > QX_P0_PAIR) return QX_ERR_INVALID_INPUT;
   c->p0_form = form;

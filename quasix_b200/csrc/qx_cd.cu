@@ -594,14 +594,23 @@ qx_ctx* make_worker(int device) {
   return c;
 }
 
+// The context's settings for its workers, `sharing` of which run at a time.
+static void worker_settings(qx_ctx* ctx, int sharing) {
+  for (qx_ctx* wk : ctx->workers) {
+    wk->p0_form = ctx->p0_form;
+    wk->contraction_form = ctx->contraction_form;
+    wk->digit_limit = ctx->digit_limit ? std::max<size_t>(1, ctx->digit_limit / sharing) : 0;
+  }
+}
+
 // Workspace estimate of one system in the grouped batch (bytes): eps of the
 // grid and of the residues, the P0 operands (split forms: hi/lo of B_ov and of
-// every chi-scaled copy), chi, B_ov^T and the pair tensors of the targets.
-static double cd_system_bytes(const qx_cd_system& s, int nw, bool tc) {
+// every chi-scaled copy; FP64: the digit operands of P0 and the contraction within
+// a worker's limit), chi, B_ov^T and the pair tensors of the targets.
+static double cd_system_bytes(const qx_cd_system& s, int nw, bool tc, size_t limit) {
   const double ldn = round_up(s.naux, 8), nov = (double)s.nocc * (s.nmo - s.nocc), ldov = round_up((int)nov, 8);
   const double eps = (nw + 2.0 * s.ntarget) * s.naux * ldn * 8.0;
-  // FP64: the digits of B_ov and of a chunk of its chi-scaled copies (k_digits.cu).
-  const double digits = 7.0 * s.naux * ldov + std::min(512.0 * 1048576, 7.0 * nw * s.naux * ldov);
+  const double digits = (double)digit_workspace_bytes(s.naux, (int)nov, s.ntarget * s.nmo, nw, limit);
   const double p0 = s.naux * ldov * 8.0 + nw * ldov * 8.0 + (tc ? (1.0 + nw) * s.naux * ldov * 4.0 : digits);
   const double pairs = (double)s.ntarget * s.nmo * ldn * (tc ? 16.0 : 8.0) + nw * (double)s.ntarget * s.nmo * 8.0;
   return eps + p0 + nov * ldn * 8.0 + pairs;
@@ -621,26 +630,26 @@ static void cd_batch_grouped(qx_ctx* ctx, qx_cd_system* systems, int nsys, int n
   const bool tc = is_tc_precision(precision);
   std::vector<int> order(nsys);
   for (int i = 0; i < nsys; ++i) order[i] = i;
+  constexpr int kWaveSystems = 64;
+  if (ctx->workers.empty()) ctx->workers.push_back(make_worker(ctx->device));
+  worker_settings(ctx, std::min(nsys, kWaveSystems));
+  const size_t limit = digit_limit(ctx->workers[0]);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-    return cd_system_bytes(systems[a], nw, tc) > cd_system_bytes(systems[b], nw, tc);
+    return cd_system_bytes(systems[a], nw, tc, limit) > cd_system_bytes(systems[b], nw, tc, limit);
   });
   constexpr double kWaveBytes = 48e9;
-  constexpr int kWaveSystems = 64;
   for (int k = 0; k < nsys;) {
     std::vector<int> wave;
     double used = 0.0;
     while (k < nsys && (int)wave.size() < kWaveSystems) {
-      const double b = cd_system_bytes(systems[order[k]], nw, tc);
+      const double b = cd_system_bytes(systems[order[k]], nw, tc, limit);
       if (!wave.empty() && used + b > kWaveBytes) break;
       wave.push_back(order[k++]);
       used += b;
     }
     const int W = (int)wave.size();
     while ((int)ctx->workers.size() < W) ctx->workers.push_back(make_worker(ctx->device));
-    for (qx_ctx* wk : ctx->workers) {
-      wk->p0_form = ctx->p0_form;
-      wk->contraction_form = ctx->contraction_form;
-    }
+    worker_settings(ctx, std::min(nsys, kWaveSystems));
     std::vector<CdProblem> probs(W);
     std::vector<CdRun> runs(W);
     std::vector<char> ok(W, 1);
@@ -828,10 +837,7 @@ extern "C" qx_status qx_g0w0_cd_batch(qx_ctx* ctx, qx_cd_system* systems, int ns
     if (nworkers < 0) nworkers = 4;
     nworkers = std::min(std::min(nworkers, 16), nsys);
     while ((int)ctx->workers.size() < nworkers) ctx->workers.push_back(make_worker(ctx->device));
-    for (qx_ctx* wk : ctx->workers) {
-      wk->p0_form = ctx->p0_form;
-      wk->contraction_form = ctx->contraction_form;
-    }
+    worker_settings(ctx, nworkers);
     // Largest systems first (P0 cost nov * naux^2 dominates), so that the
     // small ones fill in behind them.
     std::vector<int> order(nsys);

@@ -58,11 +58,14 @@ struct DevBuf {
     QX_CUDA(cudaMalloc(&ptr, n));
     bytes = n;
   }
+  void release() {
+    if (ptr) cudaFree(ptr);  // (waits for the device)
+    ptr = nullptr;
+    bytes = 0;
+  }
   template <class T>
   T* as() const { return reinterpret_cast<T*>(ptr); }
-  ~DevBuf() {
-    if (ptr) cudaFree(ptr);
-  }
+  ~DevBuf() { release(); }
 };
 
 // Grow-only page-locked host buffer: device-to-host copies into it stay
@@ -138,6 +141,9 @@ struct qx_ctx {
   // batch workers inherit it from their parent context.
   int p0_form = 0;
   int contraction_form = 0;  // QX_CONTRACT_*: tiles of the split pair contraction
+  // Bytes of the digit operands' workspace (qx_ctx_set_digit_workspace); 0: the
+  // default.  The workers of a batch share a limit in equal parts.
+  size_t digit_limit = 0;
 };
 
 namespace qx {
@@ -262,6 +268,12 @@ bool launch_eps_digits(qx_ctx* ctx, const double* bov, int ldov, int naux, int n
                        double* eps, int ldn, size_t eps_stride);
 bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc,
                                  int ldn, size_t wc_stride, int nw, double* v, int ldv);
+// Where P0 and the pair contraction take them, and the bytes of workspace that a
+// problem's two products use within a limit.
+bool digits_for_p0(int naux, int nov);
+bool digits_for_contraction(int naux);
+size_t digit_limit(const qx_ctx* ctx);
+size_t digit_workspace_bytes(int naux, int nov, int npair, int nw, size_t limit);
 // How far fixed point suits rows, by blocks of kRoughRows (k_digits.cu: rho, as the bit
 // pattern of a float; infinite rows times zero rows count as above any limit).
 constexpr int kRoughRows = 64;
