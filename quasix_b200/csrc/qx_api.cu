@@ -507,6 +507,15 @@ void validate_common(int nmo, int nocc, int naux) {
 
 using namespace qx;
 
+// The digit operands are written and read within one launcher.
+qx_ctx::qx_ctx() {
+  for (int i = 0; i < WS_COUNT; ++i) {
+    if (i >= WS_DIG_A && i <= WS_DIG_P) continue;
+    ws[i].spare = &ws[WS_DIG_A];
+    ws[i].n_spare = WS_DIG_P - WS_DIG_A + 1;
+  }
+}
+
 // A call that fails may leave setup work on the side stream reading the
 // caller's host arrays: it ends before the call returns.
 static void settle_side(qx_ctx* ctx) {

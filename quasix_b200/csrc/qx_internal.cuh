@@ -47,15 +47,22 @@ inline std::string fmt(const char* f, ...) {
   } while (0)
 
 // Device buffer owned by a context; grows, never shrinks, reused across calls.
+// What the device has no room for is tried again without the context's spare
+// buffers (n_spare of them), which hold nothing between two launchers.
 struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
+  DevBuf* spare = nullptr;
+  int n_spare = 0;
   void reserve(size_t n) {
     if (n <= bytes) return;
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-    bytes = 0;
-    QX_CUDA(cudaMalloc(&ptr, n));
+    release();
+    if (cudaMalloc(&ptr, n) != cudaSuccess) {
+      ptr = nullptr;
+      cudaGetLastError();
+      for (int i = 0; i < n_spare; ++i) spare[i].release();
+      QX_CUDA(cudaMalloc(&ptr, n));
+    }
     bytes = n;
   }
   void release() {
@@ -95,6 +102,7 @@ struct HostBuf {
 enum { QX_ST_P0 = 0, QX_ST_INV, QX_ST_CONTRACT, QX_ST_SIGMA, QX_ST_QP, QX_ST_COUNT };
 
 struct qx_ctx {
+  qx_ctx();
   int device = 0;
   int sm_count = 148;
   cudaStream_t own_stream = nullptr;

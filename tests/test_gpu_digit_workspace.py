@@ -108,6 +108,38 @@ def test_limit_holds(env):  # noqa: F811
     assert used <= (48 << 20) + 5 * (2 << 20)
 
 
+def test_operands_make_room(env):  # noqa: F811
+    """A workspace that fits the device only without the digit operands of an earlier
+    call: 120 MB and more of them are held, 90 MB are free, and the rho response of
+    40 frequencies at naux 690 takes 150 MB."""
+    import torch
+    from quasix_b200 import _native
+    rng = np.random.default_rng(6)
+    nocc, nvir, naux, nf = 2, 40, 690, 40
+    e = np.concatenate([np.linspace(-1.0, -0.5, nocc), np.linspace(0.1, 2.0, nvir)])
+    lov = rng.normal(size=(naux, nocc, nvir)) * 0.05
+    freqs = np.linspace(0.0, 2.0, nf)
+    out = np.zeros((nf, naux, naux))
+    ctx = _native.Context()
+    call = lambda n: ctx.check(ctx.lib.qx_get_rho_response(ctx.handle, n, freqs.ctypes.data, e.ctypes.data, lov.ctypes.data,
+                                                           naux, nocc, nvir, 0, out.ctypes.data))
+    call(1)
+    p0((torch, ctx), rng.normal(size=(690, 4000)), rng.uniform(0.2, 2.0, (8, 4000)))
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    hog = torch.empty(free - (90 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        call(nf)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+        ctx.close()
+    b = lov.reshape(naux, -1)
+    d = (e[:nocc, None] - e[None, nocc:]).reshape(-1)
+    ref = 4.0 * (b * (d / (freqs[-1] ** 2 + d * d))) @ b.T
+    assert np.abs(out[-1] - ref).max() < 1e-12 * np.abs(ref).max()
+
+
 def test_bad_context():
     from quasix_b200 import _native
     assert _native.load().qx_ctx_set_digit_workspace(None, 0) != 0
