@@ -495,7 +495,9 @@ bool chi_smooth(const double* energies, int nocc, int nvir, double wmax) {
   if (!eps_at_least_identity(energies, nocc, nvir, wmax / 0.9)) return false;
   const auto occ = std::minmax_element(energies, energies + nocc);
   const auto vir = std::minmax_element(energies + nocc, energies + nocc + nvir);
-  return *vir.second - *occ.first <= 64.0 * (*vir.first - *occ.second);
+  // chi' = d / (d^2 - w^2) at the smallest and at the largest transition d.
+  const double lo = *vir.first - *occ.second, hi = *vir.second - *occ.first, w2 = wmax * wmax;
+  return hi * (1.0 - w2 / (hi * hi)) <= 64.0 * lo * (1.0 - w2 / (lo * lo));
 }
 
 void validate_common(int nmo, int nocc, int naux) {

@@ -264,9 +264,9 @@ void launch_eps_fp64(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov
                      double* eps, int ldn, size_t eps_stride, int smooth);
 
 // The chi' of these energies (host array) are all positive and within a factor
-// of about 64 of each other, on the imaginary axis (wmax = 0) or for real
-// shifts up to wmax: every shift stays below 0.9 of the smallest transition and
-// the largest transition is at most 64 times the smallest.
+// of 64 of each other, on the imaginary axis (wmax = 0; the largest transition is
+// then at most 64 times the smallest) or for real shifts up to wmax, which stay
+// below 0.9 of the smallest transition.
 bool chi_smooth(const double* energies, int nocc, int nvir, double wmax);
 
 // The FP64 contractions on the integer tensor pipe (k_digits.cu); false when

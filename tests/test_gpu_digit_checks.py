@@ -157,6 +157,22 @@ def test_p0_of_rough_rows(env, N, K, rows):
     assert bad[:, 7].all() and bad[:, :, 7].all() and bad.sum() == 2 * (2 * N - 1)
 
 
+def test_p0_of_residue_weights(env):
+    """Real shifts up to 0.9 of the smallest transition, the transitions over a factor
+    of 12: weights within a factor of 64.  The bound of test_p0_of_rough_rows."""
+    rng = np.random.default_rng(8)
+    N, K = 300, 1400
+    b, d = 3.0 * rng.normal(size=(N, K)), rng.uniform(0.35, 4.2, K)
+    d[0], d[1] = 0.35, 4.2
+    chi = np.stack([4 * d / (d * d - (f * 0.35) ** 2) for f in (0.5, 0.8, 0.9)])
+    got, bl = p0(env, b, chi), b.astype(np.longdouble)
+    for w, c in enumerate(chi):
+        ref = (bl * c) @ bl.T + np.eye(N)
+        rss = np.sqrt((b * b * c * c) @ (b * b).T)
+        bound = 2.0 ** -53 * (3.5 * np.sqrt(K) * rss + (1 + np.sqrt(K)) * np.abs(ref).astype(float))
+        assert (np.abs(got[w] - ref).astype(float) - bound).max() <= 0
+
+
 @pytest.mark.parametrize("M,N,K,rows", [(256, 256, 161, "normal"), (300, 259, 170, "some opposite"),
                                         (257, 400, 301, "opposite"), (500, 256, 700, "outliers"),
                                         (256, 321, 200, "zeros")])
