@@ -271,17 +271,13 @@ struct DigitIssue {
                       ok && mbar_wait(&acc_empty[buf], ((u / dgt::NBUF) - 1) & 1, abort_flag, err, 43));
       tc_fence_after();
     }
-    // Descriptor words: 128-byte swizzle, 8-row groups 1024 bytes apart
-    // (umma_desc<64>); 32 bytes of K per MMA advance the address by 2.
-    constexpr uint32_t HI = 64u | (1u << 14) | (2u << 29);
     const uint32_t a = a0 + slot(pa) * (dgt::SLOT_BYTES >> 4);
     const uint32_t b = a0 + slot(pb) * (dgt::SLOT_BYTES >> 4) + (dgt::A_BYTES >> 4);
     const uint32_t d = tmem + buf * dgt::TN;
     if (ok && elected) {
 #pragma unroll
       for (int kk = 0; kk < dgt::BK / 32; ++kk)
-        umma_i8_pair(d, ((uint64_t)HI << 32) | (a + 2 * kk), ((uint64_t)HI << 32) | (b + 2 * kk), kDigitIdesc,
-                     start && kk == 0 ? 0u : 1u);
+        umma_i8_pair(d, umma_desc_of(a + 2 * kk), umma_desc_of(b + 2 * kk), kDigitIdesc, start && kk == 0 ? 0u : 1u);
     }
     __syncwarp();
   }
@@ -456,7 +452,7 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
     // ---------------- MMA issuer (even CTA) ----------------
     if (leader) {
       DigitIssue q;
-      q.a0 = ((smem_u32(smem) & 0x3FFFF) >> 4) | (1u << 16);
+      q.a0 = umma_desc_lo(smem_u32(smem));
       q.full = full;
       q.empty = empty;
       q.acc_full = acc_full;

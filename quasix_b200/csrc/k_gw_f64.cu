@@ -548,23 +548,21 @@ __global__ void __launch_bounds__(256) k_sweep_write(double* __restrict__ M, int
 }
 
 // After the last sweep M = -eps^-1; Wc = eps^-1 - I = -M - I.  A frequency
-// whose eps was singular gets Wc = 0 (eps^-1 replaced by the identity).  With
-// half_lower the output is W' = strict lower triangle of Wc + diag(Wc) / 2 and
-// zeros above, so that b^T Wc b = 2 b^T W' b needs only the lower triangle.
-// Row r of the finish (one block per row).
-// Rows [8 b, 8 b + 8) of the finish, one warp per row with the lanes along it
-// (a block per row left each block ~1 KB of work and the launch bound by
-// block scheduling).
+// whose eps was singular gets Wc = 0 (eps^-1 replaced by the identity).
+//
+// The half-lower finish leaves W' = strict lower triangle of Wc + diag(Wc) / 2 and
+// zeros above, so that b^T Wc b = 2 b^T W' b needs only the lower triangle: rows
+// [8 b, 8 b + 8), one warp per row with the lanes along it (a block per row left
+// each block ~1 KB of work and the launch bound by block scheduling).
 constexpr int kFinishRows = 8;
-__device__ __forceinline__ void finish_wc_rows(double* __restrict__ A, int n, int ldn, bool singular, int half_lower,
-                                               int b) {
+__device__ __forceinline__ void finish_wc_rows(double* __restrict__ A, int n, int ldn, bool singular, int b) {
   const int r = kFinishRows * b + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= n) return;
   double* row = A + (size_t)r * ldn;
   for (int c = lane; c < n; c += 32) {
     double v = 0.0;
-    if (!singular && !(half_lower && c > r)) v = -row[c] - (r == c ? 1.0 : 0.0);
-    if (half_lower && c == r) v *= 0.5;
+    if (!singular && c <= r) v = -row[c] - (r == c ? 1.0 : 0.0);
+    if (c == r) v *= 0.5;
     row[c] = v;
   }
 }
@@ -594,9 +592,9 @@ __device__ __forceinline__ void finish_wc_tile(double* __restrict__ A, int n, in
 }
 
 __global__ void __launch_bounds__(32 * kFinishRows) k_finish_wc(double* __restrict__ M, int n, int ldn, size_t stride,
-                                                               const int* __restrict__ status, int half_lower) {
+                                                               const int* __restrict__ status) {
   const int w = blockIdx.y;
-  finish_wc_rows(M + (size_t)w * stride, n, ldn, status[w] != 0, half_lower, blockIdx.x);
+  finish_wc_rows(M + (size_t)w * stride, n, ldn, status[w] != 0, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(256) k_finish_wc_full(double* __restrict__ M, int n, int ldn, size_t stride,
@@ -609,7 +607,7 @@ __global__ void __launch_bounds__(256) k_finish_wc_full(double* __restrict__ M, 
 static void launch_finish(qx_ctx* ctx, double* eps, int n, int ldn, size_t stride, int nw, const int* status,
                           int half_lower, int full) {
   if (half_lower) {
-    k_finish_wc<<<dim3(ceil_div(n, kFinishRows), nw), 256, 0, ctx->stream>>>(eps, n, ldn, stride, status, 1);
+    k_finish_wc<<<dim3(ceil_div(n, kFinishRows), nw), 256, 0, ctx->stream>>>(eps, n, ldn, stride, status);
   } else {
     const int t = ceil_div(n, 32);
     k_finish_wc_full<<<dim3(t * (t + 1) / 2, nw), 256, 0, ctx->stream>>>(eps, n, ldn, stride, status, full);
@@ -892,10 +890,10 @@ __global__ void __launch_bounds__(SweepTile::THREADS) k_gsweep_update(const GMat
 
 __global__ void __launch_bounds__(32 * kFinishRows) k_gfinish_wc(const GMat* __restrict__ mats,
                                                                  const int* __restrict__ pre, int count,
-                                                                 const int* __restrict__ status, int half_lower) {
+                                                                 const int* __restrict__ status) {
   const int g = group_of(pre, count, blockIdx.x);
   const GMat m = mats[g];
-  finish_wc_rows(m.M, m.n, m.ldn, status[g] != 0, half_lower, blockIdx.x - pre[g]);
+  finish_wc_rows(m.M, m.n, m.ldn, status[g] != 0, blockIdx.x - pre[g]);
 }
 
 __global__ void __launch_bounds__(256) k_gfinish_wc_full(const GMat* __restrict__ mats, const int* __restrict__ pre,
@@ -1067,7 +1065,7 @@ void launch_invert_wc_group(qx_ctx* ctx, const GMat* mats_in, int G, int half_lo
   }
   if (guarded) guard_end(ctx, gs);
   if (half_lower)
-    k_gfinish_wc<<<tab[off_fin + G], 256, 0, ctx->stream>>>(d_mats, d_tab + off_fin, G, status, 1);
+    k_gfinish_wc<<<tab[off_fin + G], 256, 0, ctx->stream>>>(d_mats, d_tab + off_fin, G, status);
   else
     k_gfinish_wc_full<<<tab[off_fin + G], 256, 0, ctx->stream>>>(d_mats, d_tab + off_fin, G, status);
   check_launch(ctx);

@@ -178,7 +178,7 @@ struct TcArgs {
 
 // Byte offset of the 16-bit element (row r, column c) in a 64-wide K-major
 // tile with the 128-byte swizzle (the layout TMA's SWIZZLE_128B writes into a
-// 1024-byte-aligned buffer, umma_desc<64>): rows of 128 bytes, whose 16-byte
+// 1024-byte-aligned buffer, umma_desc_lo): rows of 128 bytes, whose 16-byte
 // chunks are permuted by chunk ^ (r % 8).
 __device__ __forceinline__ uint32_t sw128_offset(int r, int c) {
   return (uint32_t)r * 128u + ((uint32_t)((c >> 3) ^ (r & 7)) << 4) + (uint32_t)(c & 7) * 2u;

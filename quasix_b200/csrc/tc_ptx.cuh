@@ -74,22 +74,6 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 
-// SM100 shared-memory matrix descriptor (version 1) for a K-major operand tile of BK 16-bit elements per row: BK = 64 uses the 128-byte
-// swizzle (layout 2, 8-row groups 1024 bytes apart), BK = 32 the 64-byte swizzle
-// (layout 4, 512 bytes apart).
-template <int BK>
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
-  static_assert(BK == 32 || BK == 64, "K block of 32 or 64 elements");
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFF) >> 4);          // start address
-  d |= (uint64_t)1 << 16;                           // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)((8 * BK * 2) >> 4) << 32;         // stride byte offset: 8 rows
-  d |= (uint64_t)1 << 46;                           // descriptor version (sm_100)
-  d |= (uint64_t)(BK == 64 ? 2 : 4) << 61;          // SWIZZLE_128B / SWIZZLE_64B
-  return d;
-}
-
-
 // An issuer of MMAs runs its loop in all 32 lanes, with the same values, and one
 // elected lane issues: the descriptors then stay in uniform registers.  With the
 // whole loop inside one lane's branch every MMA waited for its descriptors to be
@@ -100,8 +84,12 @@ __device__ __forceinline__ uint32_t elect_one() {
   asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
   return p;
 }
-// Descriptor of the operand at saddr in two words, K blocks of 64 elements
-// (umma_desc<64>): 16 elements of K advance the low word by 2.
+// SM100 shared-memory matrix descriptor (version 1) of a K-major operand tile with
+// rows of 128 bytes (64 16-bit or 128 8-bit elements of K), 128-byte swizzle: the
+// low word holds the start address and the leading byte offset (1: unused with a
+// swizzle), the high word the stride of 8 rows (1024 bytes), the version (bit 46 of
+// the whole) and the swizzle (2 in bits 61 to 63).  32 bytes of K advance the low
+// word by 2.
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFF) >> 4) | (1u << 16); }
 __device__ __forceinline__ uint64_t umma_desc_of(uint32_t lo) {
   return ((uint64_t)(64u | (1u << 14) | (2u << 29)) << 32) | lo;
