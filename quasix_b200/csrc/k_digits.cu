@@ -512,10 +512,9 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
       auto drain = [&](auto&& f) {
         if (!ok) return;
         const int buf = u & (P::NBUF - 1);
-        if (!mbar_wait(&acc_full[buf], (u / P::NBUF) & 1, abort_flag, args.err, 46)) {
-          ok = false;
-          return;
-        }
+        // The lanes leave together: what follows is collective.
+        ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (u / P::NBUF) & 1, abort_flag, args.err, 46));
+        if (!ok) return;
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * P::TN + half * P::CPW;
 #pragma unroll
