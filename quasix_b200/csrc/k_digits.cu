@@ -679,23 +679,20 @@ __global__ void __launch_bounds__(dgt::THREADS, 1)
 }
 
 // v[w][p] = 2 sum_q part[q][w][p]  (fixed order), and the items (w, block of
-// REDO_ROWS pairs) whose digits may not hold v as the DMMA kernel would: list[0 ..
-// *count), in any order.
+// REDO_ROWS pairs) that k_pair_contract_redo has to look at: list[0 .. *count), in any
+// order.
 //
 // Fixed point loses what an entry lacks of its row's bound, so the error of v is
-// not bounded by v's own terms when large entries of b meet small ones of W'
-// (exact model, K = 300: entries of b and W' graded against each other over
-// one decade 2.8, two 17, three 55, four 1100 x 2^-53 of v; FP64 sums 1 to 12).
-// With 2^e, r 2^e the bound and the norm of row b, and W, R the largest bound and
-// norm of the rows of W', the root-mean-square error of v is at most
-//   2 2^-56 r 2^e (0.58 (3 2^e R + r 2^e W) + 0.82 sqrt(K) 2^e W):
-// the entries' rounding (2^-55 / sqrt(12) of their bound) in b (twice as a factor,
-// once in the sum over n, that of the epilogue below it) and in W', and the six digit
-// products of t = 7 (each sqrt(1 / 12) 2^8 twice).  Up to 4 x 2^-53 of v it
-// stands (0.7 to 1 for a dielectric matrix and normal b of any K, 2 where an entry
-// of b is above four deviations; graded alike, over four decades, 1 to 4, where
-// the error was below 3); beyond, and where anything is not finite, the DMMA kernel
-// forms the block again.
+// not bounded by v's own terms when large entries of b meet small ones of W'.
+// With 2^e and N the bound and the norm of row b, w_n and r_n those of the rows of W',
+// K columns, the root-mean-square error of v is about
+//   2 2^-56 (0.58 2^e |b r| + 1.16 2^e N rms(r) + (0.58 N + 0.82 sqrt(K) 2^e) |b w|),
+// |b r|^2 = sum_n b_n^2 r_n^2: the entries' rounding (2^-55 / sqrt(12) of their bound)
+// in b (in C, in the sum over n, and the epilogue's below it) and in W', and the six
+// digit products of t = 7 (each sqrt(1 / 12) 2^8 twice).  Here N times the largest w
+// and r stand for the sums (most), and up to 2 x 2^-53 of the sum of the magnitudes of
+// v's half-tile sums a pair's digits stand: 1 for a dielectric matrix and normal b of
+// any K, 2 where an entry of b is above four deviations.
 constexpr int REDO_ROWS = kPairRedoRows;
 struct DigitCheck {
   const double* scale;             // [npair] 2^(e - 7)
@@ -714,12 +711,15 @@ __global__ void __launch_bounds__(256) k_digit_rowdot_sum(const double* __restri
     const int p = p0 + threadIdx.x;
     bool fail = false;
     if (p < npair) {
-      double s = 0.0;
-      for (int q = 0; q < np; ++q) s += part[((size_t)q * nw + w) * npair + p];
-      const double y = 2.0 * s;
-      v[(size_t)w * ldv + p] = y;
+      double s = 0.0, mag = 0.0;
+      for (int q = 0; q < np; ++q) {
+        const double h = part[((size_t)q * nw + w) * npair + p];
+        s += h;
+        mag += fabs(h);
+      }
+      v[(size_t)w * ldv + p] = 2.0 * s;
       const double bound = ck.scale[p] * 128.0, n2 = ck.norm[p] * bound;
-      fail = !(n2 * (0.58 * (3.0 * bound * R + n2 * W) + ck.k082 * bound * W) <= 16.0 * fabs(y));
+      fail = !(n2 * (0.58 * (3.0 * bound * R + n2 * W) + ck.k082 * bound * W) <= 16.0 * mag);
     }
     const int any = __any_sync(0xffffffffu, fail);
     if ((threadIdx.x & 31) == 0) bad[threadIdx.x >> 5] = any;
@@ -881,7 +881,7 @@ __device__ __forceinline__ void mark_rough(const RoughRows& g, int w, int r, dou
 }
 
 // What the split finds out about the rows besides their scales (each may be
-// null): norm[r], |row r| relative to 2^e, from above (the top digits' and their
+// null): norm[w lds + r], |row r| relative to 2^e, from above (the top digits' and their
 // rounding's); per batch the largest 2^e and the largest |row| (as bit patterns,
 // zero on entry; a NaN is larger than all); the marked blocks of rows.
 struct SplitStats {
@@ -946,7 +946,7 @@ __global__ void __launch_bounds__(256) k_digit_split(const double* __restrict__ 
   if (live && t == 0) {
     scale[(size_t)w * lds + r] = sc.sc;
     const double norm = (sqrt((double)squares) + 0.5 * sqrt((double)lim)) * 0x1p-7, bound = sc.sc * 128.0;
-    if (st.norm) st.norm[r] = norm;
+    if (st.norm) st.norm[(size_t)w * lds + r] = norm;
     if (st.most) {
       atomicMax(st.most + 2 * w, (unsigned long long)__double_as_longlong(bound));
       atomicMax(st.most + 2 * w + 1, (unsigned long long)__double_as_longlong(bound * norm));
@@ -1200,7 +1200,7 @@ static DigitPlan plan_contract(int npair, int naux, int nw, size_t limit, bool s
   d.fc = (int)std::max<size_t>(1, std::min<size_t>(f, nw));
   // Per pair: digits; partial sums, integers, scale, norm and list entries.
   const size_t per_p = ((size_t)2 * NT * d.fc + lds) * sizeof(double);
-  const size_t fixed_s = ((size_t)(lds + 2) * d.fc + 2) * sizeof(double);
+  const size_t fixed_s = ((size_t)(2 * lds + 2) * d.fc + 2) * sizeof(double);
   const size_t per_s = 2 * sizeof(double) + (size_t)ceil_div(d.fc, REDO_ROWS / (int)sizeof(int));
   size_t r = fixed_s < third ? std::min(limit / 4 / row, (third - fixed_s) / (per_p + per_s)) / 256 * 256 : 0;
   if (r == 0 && strict && npair > 0) {
@@ -1374,12 +1374,13 @@ bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int np
   if (!try_reserve(da, plan.a) || !try_reserve(db, plan.b) || !try_reserve(ds, plan.s) || !try_reserve(dp, plan.p))
     return false;
   int2* xt = reinterpret_cast<int2*>(dp.as<double>() + (size_t)2 * NT * fc * pc);
-  // Scales of W', its largest bounds and norms, the count of the blocks to form
-  // again (zeroed together), scales and norms of the pairs, the list of those blocks.
+  // Scales of W', its largest bounds and norms, the count of the listed blocks (zeroed
+  // together), its norms; scales and norms of the pairs, the list of blocks.
   double* sb = ds.as<double>();
   unsigned long long* most = reinterpret_cast<unsigned long long*>(sb + (size_t)lds * fc);
   int* redo_count = reinterpret_cast<int*>(most + 2 * fc);
-  double* sa = reinterpret_cast<double*>(redo_count + 2);
+  double* norm_w = reinterpret_cast<double*>(redo_count + 2);
+  double* sa = norm_w + (size_t)lds * fc;
   double* norm = sa + pc;
   int* redo = reinterpret_cast<int*>(norm + pc);
   for (int p0 = 0; p0 < npair; p0 += pc) {
@@ -1393,7 +1394,7 @@ bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int np
       if (p0 == 0 || fc < nw) {
         QX_CUDA(cudaMemsetAsync(sb, 0, ((size_t)(lds + 2) * fc + 1) * sizeof(double), ctx->stream));
         split_rows(ctx, wc + (size_t)w0 * wc_stride, naux, naux, ldn, wc_stride, n, 1, db.as<int8_t>(), ldd, sb, lds,
-                   {nullptr, most, {}});
+                   {norm_w, most, {}});
       } else {
         QX_CUDA(cudaMemsetAsync(redo_count, 0, sizeof(int), ctx->stream));
       }
@@ -1415,7 +1416,8 @@ bool launch_pair_contract_digits(qx_ctx* ctx, const double* bpt, int ldk, int np
           dp.as<double>(), 2 * NT, np, n, v + (size_t)w0 * ldv + p0, ldv, ck);
       check_launch(ctx);
       launch_pair_contract_redo(ctx, bpt + (size_t)p0 * ldk, ldk, np, naux, wc + (size_t)w0 * wc_stride, ldn, wc_stride,
-                                n, v + (size_t)w0 * ldv + p0, ldv, redo_count, redo);
+                                n, v + (size_t)w0 * ldv + p0, ldv,
+                                {redo_count, redo, sa, norm, sb, norm_w, lds, dp.as<double>(), 2 * NT});
     }
   }
   return true;

@@ -1330,17 +1330,58 @@ __global__ void __launch_bounds__(PairTile::THREADS) k_pair_contract_f64(const d
   pair_contract_block(bpt, ldk, npair, naux, wc, ldn, wc_stride, v, ldv, blockIdx.y, blockIdx.x * PairTile::BM);
 }
 
-// The blocks list[0 .. *count), w ceil(npair / BM) + block, one after the other.
+// Does fixed point hold v[w][p] of this block's pairs?  Four threads per pair form the
+// sums that the error's estimate is made of (k_digit_rowdot_sum); the digits stand up
+// to 2.5 x 2^-53 of the magnitudes of v's half-tile sums, or up to N |b r| 2^-53,
+// what FP64 sums lose of partial sums that cancel (0.5 to 0.9 of it for an
+// indefinite or nearly singular W).
+// In an exact model (estimate, digits' and FP64 sums' error in 2^-53 of those
+// magnitudes, K = 1000): dielectric matrix 1.0, 1.3, 8.2; 1000 times its norm in one
+// direction 2.6 (N |b r| 8.6), 1.2, 6.0; b graded up where W' is down, over one decade
+// 2.9, 1.7, 6.7, over one and a half 9.3, 5.5, 8.1, two 31, 11, 6.3, three 910, 86, 7.5;
+// one entry in twenty 3.3, 4.2, 1.5.
+// FP64 evGW at nmo 300 over five iterations, whose levels cross in the last two: 24.2 iter/s
+// when blocks were formed again on the first test alone, 31.4 with this one (71 of 8600
+// listed blocks), 33.1 with neither.
+__device__ __forceinline__ bool pair_digits_stand(const PairRedo& a, const double* __restrict__ bpt, int ldk, int npair,
+                                                  int naux, int nw, int w, int m0) {
+  static_assert(PairTile::THREADS == 4 * PairTile::BM, "four threads per pair");
+  const int p = min(m0 + ((int)threadIdx.x >> 2), npair - 1), t = threadIdx.x & 3;
+  const double* b = bpt + (size_t)p * ldk;
+  const double *sw = a.scale_w + (size_t)w * a.ldw, *nr = a.norm_w + (size_t)w * a.ldw;
+  double bb = 0.0, br = 0.0, bw = 0.0, rr = 0.0, mag = 0.0;
+  for (int n = t; n < naux; n += 4) {
+    const double x = b[n] * b[n], bound = 128.0 * sw[n], r = bound * nr[n];
+    bb += x;
+    rr = fma(r, r, rr);
+    br = fma(x, r * r, br);
+    bw = fma(x, bound * bound, bw);
+  }
+  for (int q = t; q < a.np; q += 4) mag += fabs(a.part[((size_t)q * nw + w) * npair + p]);
+  for (int o = 1; o <= 2; o <<= 1) {
+    bb += __shfl_xor_sync(0xffffffffu, bb, o);
+    rr += __shfl_xor_sync(0xffffffffu, rr, o);
+    br += __shfl_xor_sync(0xffffffffu, br, o);
+    bw += __shfl_xor_sync(0xffffffffu, bw, o);
+    mag += __shfl_xor_sync(0xffffffffu, mag, o);
+  }
+  const double be = 128.0 * a.scale[p], N = sqrt(bb), BR = sqrt(br), k = naux;
+  const double est =
+      0.25 * (be * (0.58 * BR + 1.16 * N * sqrt(rr / k)) + (0.58 * N + 0.82 * sqrt(k) * be) * sqrt(bw));
+  return __syncthreads_and(est <= 5.0 * mag || est <= N * BR);
+}
+
+// The listed blocks, one after the other.
 __global__ void __launch_bounds__(PairTile::THREADS) k_pair_contract_redo(const double* __restrict__ bpt, int ldk,
                                                                           int npair, int naux,
                                                                           const double* __restrict__ wc, int ldn,
-                                                                          size_t wc_stride, double* __restrict__ v,
-                                                                          int ldv, const int* __restrict__ count,
-                                                                          const int* __restrict__ list) {
-  const int n = *count, nblk = (npair + PairTile::BM - 1) / PairTile::BM;
+                                                                          size_t wc_stride, int nw,
+                                                                          double* __restrict__ v, int ldv, PairRedo redo) {
+  const int n = *redo.count, nblk = (npair + PairTile::BM - 1) / PairTile::BM;
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
-    const int it = list[i], w = it / nblk;
-    pair_contract_block(bpt, ldk, npair, naux, wc, ldn, wc_stride, v, ldv, w, (it - w * nblk) * PairTile::BM);
+    const int it = redo.list[i], w = it / nblk, m0 = (it - w * nblk) * PairTile::BM;
+    if (pair_digits_stand(redo, bpt, ldk, npair, naux, nw, w, m0)) continue;
+    pair_contract_block(bpt, ldk, npair, naux, wc, ldn, wc_stride, v, ldv, w, m0);
   }
 }
 
@@ -1355,12 +1396,12 @@ static void pair_attributes_once(int device) {
 
 // Two blocks per SM go through the list; an empty one costs the launch.
 void launch_pair_contract_redo(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc, int ldn,
-                               size_t wc_stride, int nw, double* v, int ldv, const int* count, const int* list) {
+                               size_t wc_stride, int nw, double* v, int ldv, const PairRedo& redo) {
   using T = PairTile;
   pair_attributes_once(ctx->device);
   const long long items = (long long)ceil_div(npair, T::BM) * nw;
   k_pair_contract_redo<<<(unsigned)std::min<long long>(items, 2 * ctx->sm_count), T::THREADS, T::SMEM, ctx->stream>>>(
-      bpt, ldk, npair, naux, wc, ldn, wc_stride, v, ldv, count, list);
+      bpt, ldk, npair, naux, wc, ldn, wc_stride, nw, v, ldv, redo);
   check_launch(ctx);
 }
 

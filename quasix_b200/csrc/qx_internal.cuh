@@ -292,11 +292,22 @@ __device__ __forceinline__ bool rough_tile(unsigned a, unsigned b, float limit) 
 // blocks' rho, rough[w ceil(naux / kRoughRows) + block], is above the limit.
 void launch_eps_dmma(qx_ctx* ctx, const double* bov, int ldov, int naux, int nov, const double* chi, int nw, double* eps,
                      int ldn, size_t eps_stride, const unsigned* rough, float rough_limit);
-// The DMMA contraction of the listed blocks of kPairRedoRows pairs (device list and
-// count), which the digits may not hold.
+// The DMMA contraction of those of the listed blocks of kPairRedoRows pairs that the
+// digits do not hold, by the error's estimate for each pair.
 constexpr int kPairRedoRows = 64;
+struct PairRedo {
+  const int* count;        // blocks listed
+  const int* list;         // w ceil(npair / kPairRedoRows) + block
+  const double* scale;     // [npair] 2^(e - 7) of the pairs' rows
+  const double* norm;      // [npair] their norms relative to 2^e
+  const double* scale_w;   // [nw][ldw] the same of the rows of W'
+  const double* norm_w;
+  int ldw;
+  const double* part;      // [np][nw][npair] half-tile sums
+  int np;
+};
 void launch_pair_contract_redo(qx_ctx* ctx, const double* bpt, int ldk, int npair, int naux, const double* wc, int ldn,
-                               size_t wc_stride, int nw, double* v, int ldv, const int* count, const int* list);
+                               size_t wc_stride, int nw, double* v, int ldv, const PairRedo& redo);
 bool gemm_nt_digits(qx_ctx* ctx, const double* A, int M, int lda, const double* B, int N, int ldb, int K, double* C,
                     int ldc);
 

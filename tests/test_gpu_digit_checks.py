@@ -90,6 +90,24 @@ def test_contraction_of_opposite_grading(env, K, P, decades):
     assert (np.abs((again - ref) / ref).astype(float)[:, keep] * 2.0 ** 53).max() < 6 * np.sqrt(K / 2) + 24
 
 
+@pytest.mark.parametrize("K,big", [(200, 0.0), (200, 1e3), (500, 1e3), (500, 1e6)])
+def test_contraction_of_indefinite_matrices(env, K, big):
+    """Wigner matrices, and `big` in one direction: the digits stand up to the rounding
+    of FP64 partial sums, of which N |b r| 2^-53 is the estimate (k_gw_f64.cu); six
+    deviations of either, or of the K / 2 roundings of v's own sums."""
+    rng = np.random.default_rng(K)
+    u, b = rng.normal(size=K) / np.sqrt(K), rng.normal(size=(130, K))
+    w = rng.normal(size=(2, K, K)) / np.sqrt(K)
+    w = w + w.transpose(0, 2, 1) - big * np.outer(u, u)
+    wl = np.stack([np.tril(x, -1) + np.diag(np.diag(x)) / 2 for x in w])
+    got, ref = contract(env, b, wl), contract_exact(b, wl)
+    for k in range(2):
+        c = b * (b @ wl[k].T)
+        mag = sum(2 * np.abs(c[:, q:q + 64].sum(1)) for q in range(0, K, 64))
+        nbr = np.linalg.norm(b, axis=1) * np.sqrt((b * b) @ (wl[k] ** 2).sum(1))
+        assert (np.abs(got[k] - ref[k]).astype(float) <= 2.0 ** -53 * 6 * (nbr + np.sqrt(K / 2) * mag)).all()
+
+
 def test_contraction_of_zeros(env):
     rng = np.random.default_rng(1)
     wl = definite(rng, 200, np.ones(200), 2)
