@@ -13,25 +13,28 @@
 // K. Ozaki et al., Numer. Algorithms 59 (2012) 95) and added up in 64-bit
 // integers, then in FP64.  What is lost is the rounding of each entry to 2^-56
 // of its row's bound and the digit products of t >= 7; no FP64 rounding
-// occurs inside the sum over k, whereas the DMMA kernels round once every four k.
+// occurs inside the sum over k, whereas the DMMA kernels err like one rounding per
+// k.  Rows that this does not suit are noticed, and their products formed by the
+// DMMA kernels (RoughRows, k_digit_rowdot_sum).
 //
 // Why: a DGEMM on the FP64 tensor pipe peaks at 35 TFLOP/s here; the integer
 // pipe does the 28 products of digits at up to 4.5 POP/s.  At nmo 300 / naux 1000
-// / 32 frequencies the contraction of all 45 150 pairs takes 14.4 ms (DMMA: 52.8
-// ms) and P0 3.9 ms (13.0 ms) plus 0.8 ms for its digits; P0's tiles keep the
-// tensor pipe busy for 90 % of the cycles, at the 1.6 GHz that the power limit
-// leaves.  P0's error is 2 to 6 x 2^-53 of the root-sum-square of the terms of
-// an element from K = 200 to 17 500, the DMMA kernel's 3 to 29.
+// / 32 frequencies the contraction of all 45 150 pairs takes 15.0 ms (DMMA: 52.8
+// ms) and P0 3.9 ms (13.0 ms) plus 0.9 ms for its digits; the tensor pipe is busy for
+// 93 % of an SM's active cycles in P0 and 83 % in the contraction (a small case of each),
+// at the 1.65 GHz that the power limit leaves.  P0's error is 4.6 to 7.1 x 2^-53 of
+// the root-sum-square of the terms of an element from K = 1024 to 10 400, the DMMA
+// kernel's 8.5 to 28.
 //
 // The kernel runs on CTA pairs (cta_group::2, M = 256, N = 128).  Why this
 // tile: the seven accumulators of a tile are formed in two passes over K, D_4
 // to D_6 and then D_3 to D_0 (4 x 128 columns fill TMEM), so that a digit
-// slice loaded once per K block feeds up to seven products: 36 bytes per SM
-// and cycle of MMA from L2, where one product per load would need 96.  Slices
+// slice loaded once per K block feeds up to seven products: 35 to 37 bytes per SM
+// and cycle from L2, where one product per load would need 96.  Slices
 // travel through a ring of nine 24 KB slots (this CTA's 128 rows of A and half
 // of the B tile, 128 bytes of K each), in an order that lets early slices leave
-// while late ones arrive.  (64-byte slices leave room for two whole blocks, but
-// the tensor pipe then ran at 68 % instead of 90 % of its cycles.)  The
+// while late ones arrive (64-byte slices leave room for two whole blocks, but
+// measured slower).  The
 // accumulators end their sums one after the other, and each is handed to the
 // epilogue at once, so that the four buffers go round without the MMAs
 // waiting for a drain.  The epilogue keeps the 64-bit sums of its 128 x 128 tile
